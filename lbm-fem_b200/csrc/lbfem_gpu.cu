@@ -9,6 +9,7 @@
 #include "contraction_study.cuh"
 #include "quad.cuh"
 #include "batch_group.cuh"
+#include "cg_fused.cuh"
 
 #include <cuda_runtime.h>
 
@@ -273,6 +274,14 @@ namespace
     return LBFEM_OK;
   }
 
+  template <int P, bool SEP>
+  int
+  set_fused(lbfem_gpu_ctx *ctx)
+  {
+    CK(cudaFuncSetAttribute(k_cg_fused<P, SEP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)); // 16 CTAs
+    return set_smem(ctx, k_cg_fused<P, SEP>, 200 * 1024);
+  }
+
   template <int P>
   int
   set_smem_attributes(lbfem_gpu_ctx *ctx)
@@ -308,6 +317,7 @@ namespace
         (st = set_smem(ctx, kg_stream_pair<P, PAIR_LEELIN>, pair_smem<P, PAIR_LEELIN>())) ||
         (st = set_smem(ctx, kg_stream_pair<P, PAIR_BARDOW>, pair_smem<P, PAIR_BARDOW>())) ||
         (st = set_smem(ctx, kg_window<P>, window_smem<P>())) ||
+        (st = set_fused<P, false>(ctx)) || (st = set_fused<P, true>(ctx)) ||
         (st = set_smem(ctx, k_richardson_pass<P, double>, cg_smem<P, double>(0))) ||
         (st = set_smem(ctx, k_richardson_pass<P, float>, cg_smem<P, float>(0))))
       return st;
@@ -739,6 +749,125 @@ namespace
     return LBFEM_OK;
   }
 
+  // ------------------------------------------------ the solve in one launch
+  // How k_cg_fused runs a solve of this context, if it does (group > 0): one cluster of
+  // `group` CTAs per system.
+  struct FusedPlan
+  {
+    int group = 0, threads = 0;
+    size_t smem = 0;
+    int n = 0, sys[NM] = {};
+    bool sep = false;
+  };
+
+  // The solve runs in one launch when its operator is a product (the mass matrix, or the
+  // TG3 matrix of axis-parallel directions) and a system fits in a cluster: its
+  // shared memory, and a thread's share of the nodes in its registers. Clusters of 8
+  // CTAs of up to 512 threads, one CTA per SM, of which 15 are resident at once; else
+  // of 16 CTAs of up to 256 threads, which must fit an SM in pairs (7 clusters of 16
+  // are resident with one CTA per SM, 14 with two). Measured per step, FP64 Bardow at
+  // tolerance 1e-10, clusters of 8 / of 16 / the loop of kernels: 64^2 Q1 85 / 89 /
+  // 226 us, 180^2 Q1 105 / 109 / 193 us, 64^2 Q2 162 / 177 / 458 us, 32^2 Q4 157 /
+  // 168 / 450 us.
+  FusedPlan
+  fused_plan(const lbfem_gpu_ctx *ctx, const CgCall &c)
+  {
+    FusedPlan f;
+    if (ctx->strip || ctx->distorted || c.opk == OPK_LAPLACE)
+      return f;
+    f.sep = c.opk == OPK_TG3;
+    for (int s = 0; s < c.nsys; ++s)
+      if (!((c.skip >> s) & 1))
+        {
+          if (f.sep && c.sc.kxy[s] != 0.)
+            return f;
+          f.sys[f.n++] = s;
+        }
+    if (f.n == 0)
+      return f;
+    const Grid &g = ctx->grid;
+    with_degree(ctx->P, [&](auto PP) -> int {
+      constexpr int P = decltype(PP)::value;
+      using S = FusedShape<P>;
+      for (const int group : {8, 16})
+        {
+          const int most = group == 8 ? S::THREADS : S::THREADS / 2;
+          const int ncr = (g.ncy + group - 1) / group; // the most cell rows of a band, the last one included
+          const size_t bytes = sizeof(double) * size_t(fused_smem_doubles<P>(g.nfx, g.ncx, ncr));
+          const long long tasks = (long long)(ncr + 1) * g.nfx;
+          if (group > g.ncy || bytes > size_t(group == 8 ? 200 : 100) * 1024 || tasks > (long long)S::MAXT * most)
+            continue;
+          f.group = group;
+          f.threads = int(std::min<long long>(most, (tasks + 31) / 32 * 32));
+          f.smem = bytes;
+          break;
+        }
+      return 0;
+    });
+    return f;
+  }
+
+  template <int P, bool SEP>
+  cudaError_t
+  fused_launch(const FusedPlan &f, const Geo &geo, const FusedArgs &a, cudaStream_t stream)
+  {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(f.group * f.n);
+    lc.blockDim = dim3(f.threads);
+    lc.dynamicSmemBytes = f.smem;
+    lc.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = f.group;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k_cg_fused<P, SEP>, geo, a);
+  }
+
+  // The solve c in one launch (plan f): x <- A^{-1} b. ds: the counters of a graph-launched step.
+  int
+  fused_solve(lbfem_gpu_ctx *ctx, const FusedPlan &f, CgState *state, const CgCall &c, DevStats *ds)
+  {
+    FusedArgs a{};
+    a.b = c.b;
+    a.x_cur = c.x_cur;
+    a.x_prev = c.x_prev;
+    a.x = c.x_new;
+    a.st = state;
+    a.ds = ds;
+    a.sc = c.sc;
+    for (int k = 0; k < f.n; ++k)
+      a.sys[k] = f.sys[k];
+    a.extrapolate = c.extrapolate;
+    a.group = f.group;
+    a.cg_tol = c.tol >= 0 ? c.tol : ctx->prm.cg_tolerance;
+    a.max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
+    const Geo geo = geo_of(ctx);
+    CK(cudaMemsetAsync(state, 0, sizeof(CgState), ctx->stream));
+    return with_degree(ctx->P, [&](auto PP) -> int {
+      constexpr int P = decltype(PP)::value;
+      CK((f.sep ? fused_launch<P, true>(f, geo, a, ctx->stream) : fused_launch<P, false>(f, geo, a, ctx->stream)));
+      ++ctx->launches;
+      return LBFEM_OK;
+    });
+  }
+
+  // The status code of a CG solve that ended with CgState status s.
+  int
+  cg_status(lbfem_gpu_ctx *ctx, int s, int max_its)
+  {
+    switch (s)
+      {
+        case 0:
+          return LBFEM_OK;
+        case 3:
+          return fail(ctx, LBFEM_ERR_NONFINITE, "CG: non-finite residual");
+        default:
+          return fail(ctx, LBFEM_ERR_NO_CONVERGENCE, "CG: iteration cap %d reached", max_its);
+      }
+  }
+
   // Jacobi-PCG in the order of updates of deal.II SolverCG (mass.h:204-211),
   // host-driven, with the work buffers w. *its_out: CG iterations summed over
   // the systems.
@@ -748,8 +877,27 @@ namespace
     const double tol = c.tol >= 0 ? c.tol : ctx->prm.cg_tolerance;
     const int max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
     const int nsys = c.nsys;
-    CK(cudaMemsetAsync(w.state, 0, sizeof(CgState), ctx->stream));
     int n_tiles = 0, st;
+    const FusedPlan f = w.state == ctx->d_cg ? fused_plan(ctx, c) : FusedPlan{};
+    if (f.group)
+      {
+        if ((st = fused_solve(ctx, f, w.state, c, nullptr)))
+          return st;
+        CK(cudaMemcpyAsync(ctx->h_cg, w.state, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (ctx->trace)
+          {
+            std::fprintf(stderr, "lbfem cg: one launch, it (res/tol)");
+            for (int q = 0; q < nsys; ++q)
+              std::fprintf(stderr, " %d (%.2e)", ctx->h_cg->it[q],
+                           ctx->h_cg->tol[q] > 0 ? ctx->h_cg->res[q] / ctx->h_cg->tol[q] : 0.0);
+            std::fprintf(stderr, "\n");
+          }
+        if (its_out)
+          *its_out = ctx->h_cg->total_its;
+        return cg_status(ctx, ctx->h_cg->status, max_its);
+      }
+    CK(cudaMemsetAsync(w.state, 0, sizeof(CgState), ctx->stream));
     if ((st = cg_launch_start(ctx, w, c, &n_tiles)) || (st = reduce_into(ctx, w.partials, w.sums, n_tiles, 3 * NM)) ||
         (st = strip_allreduce(ctx, 3 * NM)))
       return st;
@@ -787,11 +935,7 @@ namespace
       }
     if (its_out)
       *its_out = ctx->h_cg->total_its;
-    if (ctx->h_cg->status == 2)
-      return fail(ctx, LBFEM_ERR_NO_CONVERGENCE, "CG: iteration cap %d reached", max_its);
-    if (ctx->h_cg->status == 3)
-      return fail(ctx, LBFEM_ERR_NONFINITE, "CG: non-finite residual");
-    return LBFEM_OK;
+    return cg_status(ctx, ctx->h_cg->status, max_its);
   }
 
   CgScratch<double>
@@ -1635,6 +1779,12 @@ namespace
     const double tol = c.tol >= 0 ? c.tol : ctx->prm.cg_tolerance;
     const int max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
     const CgScratch<double> w = ctx_scratch(ctx);
+    const FusedPlan f = fused_plan(ctx, c);
+    if (f.group)
+      {
+        *body_kernels = 0;
+        return fused_solve(ctx, f, w.state, c, ctx->d_stats);
+      }
     cudaStreamCaptureStatus cs;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamGetCaptureInfo_v3(ctx->stream, &cs, nullptr, &graph, nullptr, nullptr, nullptr));
@@ -1923,9 +2073,7 @@ namespace
         const double tol = ctx->mixed ? mixed_tolerance(ctx->prm) : ctx->prm.cg_tolerance;
         if (ctx->mixed)
           return mixed_status(ctx, after.sticky, tol);
-        if (after.sticky == 3)
-          return fail(ctx, LBFEM_ERR_NONFINITE, "CG: non-finite residual");
-        return fail(ctx, LBFEM_ERR_NO_CONVERGENCE, "CG: iteration cap %d reached", ctx->prm.cg_max_iterations);
+        return cg_status(ctx, after.sticky, ctx->prm.cg_max_iterations);
       }
     return LBFEM_OK;
   }
