@@ -274,34 +274,12 @@ namespace
     return LBFEM_OK;
   }
 
-  template <int P, bool SEP>
-  int
-  set_fused(lbfem_gpu_ctx *ctx)
-  {
-    CK(cudaFuncSetAttribute(k_cg_fused<P, SEP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)); // 16 CTAs
-    return set_smem(ctx, k_cg_fused<P, SEP>, 200 * 1024);
-  }
-
   template <int P>
   int
   set_smem_attributes(lbfem_gpu_ctx *ctx)
   {
     int st;
-    if ((st = set_smem(ctx, k_advection<P, ADV_TG, double>, advection_smem<P, ADV_TG, double>())) ||
-        (st = set_smem(ctx, k_advection<P, ADV_TG_COLLIDE, double>, advection_smem<P, ADV_TG_COLLIDE, double>())) ||
-        (st = set_smem(ctx, k_advection<P, ADV_LEELIN_FEQ, double>, advection_smem<P, ADV_LEELIN_FEQ, double>())) ||
-        (st = set_smem(ctx, k_advection<P, ADV_LEELIN_FUSED, double>, advection_smem<P, ADV_LEELIN_FUSED, double>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_LEELIN>, pair_smem<P, PAIR_LEELIN>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_BARDOW>, pair_smem<P, PAIR_BARDOW>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_LEELIN, TileShapeAlt<P>>,
-                       pair_smem<P, PAIR_LEELIN, TileShapeAlt<P>>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_BARDOW, TileShapeAlt<P>>,
-                       pair_smem<P, PAIR_BARDOW, TileShapeAlt<P>>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_LEELIN, TileShapeSmall<P>>,
-                       pair_smem<P, PAIR_LEELIN, TileShapeSmall<P>>())) ||
-        (st = set_smem(ctx, k_stream_pair<P, PAIR_BARDOW, TileShapeSmall<P>>,
-                       pair_smem<P, PAIR_BARDOW, TileShapeSmall<P>>())) ||
-        (st = set_smem(ctx, k_mass_vmult<P>, cg_smem<P, double>(0))) ||
+    if ((st = set_smem(ctx, k_mass_vmult<P>, cg_smem<P, double>(0))) ||
         (st = set_smem(ctx, k_cg_start<P, double, double, double>, cg_smem<P, double>(1))) ||
         (st = set_smem(ctx, k_cg_p<P, double>, cg_smem<P, double>(0))) ||
         (st = set_smem(ctx, k_cg_update<P, double>, cg_smem<P, double>(0))) ||
@@ -317,7 +295,6 @@ namespace
         (st = set_smem(ctx, kg_stream_pair<P, PAIR_LEELIN>, pair_smem<P, PAIR_LEELIN>())) ||
         (st = set_smem(ctx, kg_stream_pair<P, PAIR_BARDOW>, pair_smem<P, PAIR_BARDOW>())) ||
         (st = set_smem(ctx, kg_window<P>, window_smem<P>())) ||
-        (st = set_fused<P, false>(ctx)) || (st = set_fused<P, true>(ctx)) ||
         (st = set_smem(ctx, k_richardson_pass<P, double>, cg_smem<P, double>(0))) ||
         (st = set_smem(ctx, k_richardson_pass<P, float>, cg_smem<P, float>(0))))
       return st;
@@ -370,6 +347,23 @@ namespace
   int quad_solve(lbfem_gpu_ctx *ctx, const double *b, double *x, int nsys, int64_t *its);
   int quad_vmult(lbfem_gpu_ctx *ctx, const double *x, double *y, int nsys);
 
+  // How many CTAs share the populations of a streaming tile: the largest power of two up
+  // to `most` at which all CTAs still run at once (two on each of 148 SMs). A tile's
+  // CTA works through its populations one after the other, so a mesh of few tiles is
+  // bound by that chain, while a split tile's CTAs each form the moments again.
+  // Measured, FP64 lumped step with 1 / 2 / 4 / 8 CTAs per tile: 18 tiles 63 / 47 /
+  // 39 / 34 us, 55 tiles 63 / 47 / 41 / 46, 96 tiles 65 / 54 / 59 / 61, 260 tiles 73 /
+  // 80 / 92 / 113; FP32 pairs with 1 / 2 / 4: 17 tiles 30 / 26 / 24 us, 152 tiles 43 /
+  // 47 / 52.
+  int
+  split_of(const dim3 &tiles, int most)
+  {
+    int z = 1;
+    while (z < most && int(tiles.x * tiles.y) * 2 * z <= 2 * 148)
+      z *= 2;
+    return z;
+  }
+
   // ds: the step counters of a step (its kernel does nothing after a failure), null otherwise.
   template <typename R>
   int
@@ -386,26 +380,31 @@ namespace
     const Geo geo = geo_of(ctx);
     return with_degree(ctx->P, [&](auto PP) -> int {
       constexpr int P = decltype(PP)::value;
-      const dim3 grid = tile_grid<P>(ctx->grid);
+      dim3 grid = tile_grid<P>(ctx->grid);
+      grid.z = split_of(grid, NM);
+      auto run = [&](auto MODE, auto SPLIT) -> cudaError_t {
+        constexpr int M = decltype(MODE)::value;
+        auto kernel = k_advection<P, M, R, decltype(SPLIT)::value>;
+        constexpr size_t smem = advection_smem<P, M, R>();
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e == cudaSuccess)
+          kernel<<<grid, THREADS, smem, ctx->stream>>>(geo, ds, f, feq, fout, rhs, ac);
+        return e;
+      };
+      auto pick = [&](auto MODE) { return grid.z > 1 ? run(MODE, std::true_type()) : run(MODE, std::false_type()); };
       switch (mode)
         {
           case ADV_TG:
-            if constexpr (sizeof(R) == sizeof(double))
-              k_advection<P, ADV_TG, R>
-                <<<grid, THREADS, advection_smem<P, ADV_TG, R>(), ctx->stream>>>(geo, ds, f, feq, fout, rhs, ac);
+            CK(pick(std::integral_constant<int, ADV_TG>()));
             break;
           case ADV_TG_COLLIDE:
-            k_advection<P, ADV_TG_COLLIDE, R>
-              <<<grid, THREADS, advection_smem<P, ADV_TG_COLLIDE, R>(), ctx->stream>>>(geo, ds, f, feq, fout, rhs, ac);
+            CK(pick(std::integral_constant<int, ADV_TG_COLLIDE>()));
             break;
           case ADV_LEELIN_FEQ:
-            if constexpr (sizeof(R) == sizeof(double))
-              k_advection<P, ADV_LEELIN_FEQ, R>
-                <<<grid, THREADS, advection_smem<P, ADV_LEELIN_FEQ, R>(), ctx->stream>>>(geo, ds, f, feq, fout, rhs, ac);
+            CK(pick(std::integral_constant<int, ADV_LEELIN_FEQ>()));
             break;
           default:
-            k_advection<P, ADV_LEELIN_FUSED, R>
-              <<<grid, THREADS, advection_smem<P, ADV_LEELIN_FUSED, R>(), ctx->stream>>>(geo, ds, f, feq, fout, rhs, ac);
+            CK(pick(std::integral_constant<int, ADV_LEELIN_FUSED>()));
         }
       LAUNCHED();
       return LBFEM_OK;
@@ -427,20 +426,23 @@ namespace
       auto go = [&](auto SS) {
         using S = decltype(SS);
         using T = Tile<P, S>;
-        const dim3 grid((ctx->grid.nfx + T::TX - 1) / T::TX, (ctx->grid.nfy + T::TY - 1) / T::TY);
-        if (mode == PAIR_BARDOW)
-          k_stream_pair<P, PAIR_BARDOW, S><<<grid, THREADS, pair_smem<P, PAIR_BARDOW, S>(), ctx->stream>>>(
-            geo, ds, d, dout, rhs, ac);
-        else
-          k_stream_pair<P, PAIR_LEELIN, S><<<grid, THREADS, pair_smem<P, PAIR_LEELIN, S>(), ctx->stream>>>(
-            geo, ds, d, dout, rhs, ac);
+        dim3 grid((ctx->grid.nfx + T::TX - 1) / T::TX, (ctx->grid.nfy + T::TY - 1) / T::TY);
+        grid.z = split_of(grid, 4);
+        auto run = [&](auto MODE, auto SPLIT) -> cudaError_t {
+          constexpr int M = decltype(MODE)::value;
+          auto kernel = k_stream_pair<P, M, S, decltype(SPLIT)::value>;
+          constexpr size_t smem = pair_smem<P, M, S>();
+          const cudaError_t e =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+          if (e == cudaSuccess)
+            kernel<<<grid, THREADS, smem, ctx->stream>>>(geo, ds, d, dout, rhs, ac);
+          return e;
+        };
+        auto pick = [&](auto MODE) { return grid.z > 1 ? run(MODE, std::true_type()) : run(MODE, std::false_type()); };
+        return mode == PAIR_BARDOW ? pick(std::integral_constant<int, PAIR_BARDOW>())
+                                   : pick(std::integral_constant<int, PAIR_LEELIN>());
       };
-      if (shape == 1)
-        go(TileShapeAlt<P>{});
-      else if (shape == 2)
-        go(TileShapeSmall<P>{});
-      else
-        go(TileShape<P>{});
+      CK((shape == 1 ? go(TileShapeAlt<P>{}) : shape == 2 ? go(TileShapeSmall<P>{}) : go(TileShape<P>{})));
       LAUNCHED();
       return LBFEM_OK;
     });
@@ -811,6 +813,13 @@ namespace
   cudaError_t
   fused_launch(const FusedPlan &f, const Geo &geo, const FusedArgs &a, cudaStream_t stream)
   {
+    // set here and not when a context is made: only the solves of small meshes load the kernel
+    auto kernel = k_cg_fused<P, SEP>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.smem));
+    if (e == cudaSuccess && f.group > 8)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess)
+      return e;
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(f.group * f.n);
     lc.blockDim = dim3(f.threads);
@@ -822,7 +831,7 @@ namespace
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     lc.attrs = &at;
     lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, k_cg_fused<P, SEP>, geo, a);
+    return cudaLaunchKernelEx(&lc, kernel, geo, a);
   }
 
   // The solve c in one launch (plan f): x <- A^{-1} b. ds: the counters of a graph-launched step.

@@ -744,7 +744,10 @@ namespace lbfem_gpu
   // 0 (constrained rows, as distribute_local_to_global leaves them).
   // R = double: populations f; R = float: deviations f - w (the operator
   // annihilates constants, and collide / feq are applied in deviation form).
-  template <int P, int MODE, typename R>
+  // SPLIT: grid.z CTAs share the 8 moving populations of a tile (split_of); every CTA
+  // forms the moments, the first one also takes the rest population and the images.
+  // A population's arithmetic does not depend on the split.
+  template <int P, int MODE, typename R, bool SPLIT = false>
   __global__ void __launch_bounds__(THREADS, 2)
     k_advection(const Geo geo, const DevStats *__restrict__ ds, const R *__restrict__ f, const R *__restrict__ feq,
                 R *__restrict__ fout, R *__restrict__ rhs, const AdvCoef ac)
@@ -846,7 +849,9 @@ namespace lbfem_gpu
     const int by_lo = g.py ? -1 : 0, by_hi = g.py ? -1 : g.nfy - 1;
     const R omega = R(ac.omega);
 
-    for (int a = (MODE == ADV_TG_COLLIDE ? 0 : 1); a < Q; ++a)
+    const int z = SPLIT ? blockIdx.z : 0;
+    const int a_lo = SPLIT ? 1 + z * (NM / gridDim.z) : 1, a_hi = SPLIT ? a_lo + NM / gridDim.z : Q;
+    for (int a = (MODE == ADV_TG_COLLIDE && z == 0 ? 0 : a_lo); a < a_hi; ++a)
       {
         __syncthreads(); // the previous population's passes are done with s_u / s_y
         stage<P>(s_u, maps, [&](long long idx) { return f[a * N + idx]; });
@@ -934,6 +939,8 @@ namespace lbfem_gpu
 
     if constexpr (MODE == ADV_TG_COLLIDE)
       {
+        if (z != 0)
+          return;
         // the images collide their own (stale) populations, as the nodal map does
         for (int t = threadIdx.x; t < T::TY * T::TX; t += blockDim.x)
           {

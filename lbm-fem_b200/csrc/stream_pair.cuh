@@ -386,16 +386,19 @@ namespace lbfem_gpu
   // pair by pair; PAIR_BARDOW also writes the collided deviations g* to dout.
   // Images get r = 0 (constrained rows).
   // The tile (bx, by) of the kernel below (also the body of its batched form, one
-  // launch over the tiles of many instances).
-  template <int P, int MODE, typename S>
+  // launch over the tiles of many instances), for the pairs split_lo .. split_hi - 1 if
+  // SPLIT; the call with the first pair also takes the rest population and the images.
+  template <int P, int MODE, typename S, bool SPLIT = false>
   __device__ __forceinline__ void
   stream_pair_tile(const Geo &geo, const DevStats *__restrict__ ds, const float *__restrict__ d,
-                   float *__restrict__ dout, float *__restrict__ rhs, const AdvCoef &ac, int bx, int by)
+                   float *__restrict__ dout, float *__restrict__ rhs, const AdvCoef &ac, int bx, int by,
+                   int split_lo = 0, int split_hi = 4)
   {
     if (ds && ds->sticky)
       return; // a step after a failed solve: the populations must stay as they are
     using T = Tile<P, S>;
     constexpr bool BARDOW = MODE == PAIR_BARDOW;
+    const int pr_lo = SPLIT ? split_lo : 0, pr_hi = SPLIT ? split_hi : 4;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     float2 *s_pb = reinterpret_cast<float2 *>(sm_raw);        // [2][NF] the pair, double-buffered
     float2 *s_y = s_pb + 2 * T::NF;                           // [3][NY] x-pass outputs
@@ -457,7 +460,7 @@ namespace lbfem_gpu
         }
       cp_async_commit();
     };
-    issue_pair(0);
+    issue_pair(pr_lo);
 
     // moments of every footprint node (Lee-Lin: wall velocity imposed, and the
     // even equilibrium base drho - 1.5 rho u.u; Bardow: the node's own moments
@@ -526,7 +529,7 @@ namespace lbfem_gpu
     const int by_lo = g.py ? -1 : 0, by_hi = g.py ? -1 : g.nfy - 1;
     const float omega = float(ac.omega);
 
-    if constexpr (BARDOW)
+    if (BARDOW && pr_lo == 0)
       {
         // the rest population: collide only (no streaming)
         __syncthreads();
@@ -544,13 +547,13 @@ namespace lbfem_gpu
           }
       }
 
-    for (int pr = 0; pr < 4; ++pr)
+    for (int pr = pr_lo; pr < pr_hi; ++pr)
       {
         const int a = pr + 1, ab = pr + 5; // opposite populations
         const float *pk = ac.pk[pr];
         const float ex = pk[2], ey = pk[4], w = ac.pw[pr], wl = ac.pwl[pr];
         float2 *s_u = s_pb + (pr & 1) * T::NF;
-        if (pr < 3)
+        if (pr + 1 < pr_hi)
           {
             issue_pair(pr + 1); // its buffer was last read by the x pass of pair pr - 1
             cp_async_wait_group<1>();
@@ -643,7 +646,7 @@ namespace lbfem_gpu
           }
       }
 
-    if constexpr (BARDOW)
+    if (BARDOW && pr_lo == 0)
       {
         // the images collide their own (stale) populations, as the nodal map does
         for (int t = threadIdx.x; t < T::TY * T::TX; t += blockDim.x)
@@ -665,11 +668,20 @@ namespace lbfem_gpu
       }
   }
 
-  template <int P, int MODE, typename S = TileShape<P>>
+  // SPLIT: grid.z CTAs share the four pairs of a tile (split_of); unsplit, the pair loop
+  // has a constant count, which is 5 to 10% faster.
+  template <int P, int MODE, typename S = TileShape<P>, bool SPLIT = false>
   __global__ void __launch_bounds__(THREADS, S::MIN_CTAS)
     k_stream_pair(const Geo geo, const DevStats *__restrict__ ds, const float *__restrict__ d,
                   float *__restrict__ dout, float *__restrict__ rhs, const AdvCoef ac)
   {
-    stream_pair_tile<P, MODE, S>(geo, ds, d, dout, rhs, ac, blockIdx.x, blockIdx.y);
+    if constexpr (SPLIT)
+      {
+        const int per_z = 4 / gridDim.z;
+        stream_pair_tile<P, MODE, S, true>(geo, ds, d, dout, rhs, ac, blockIdx.x, blockIdx.y, blockIdx.z * per_z,
+                                           (blockIdx.z + 1) * per_z);
+      }
+    else
+      stream_pair_tile<P, MODE, S>(geo, ds, d, dout, rhs, ac, blockIdx.x, blockIdx.y);
   }
 } // namespace lbfem_gpu
