@@ -258,7 +258,7 @@ int lbfem_gpu_predictor_corrector(lbfem_gpu_ctx *ctx, double *f, const double *f
  * `stream` before the call, and the work queued on `stream` after the call
  * waits for it (events; the host does not wait). The exceptions are
  * lbfem_gpu_mass_solve_dev with consistent mass, whose Jacobi-PCG reads its
- * state back once per iteration and returns when the solve is done, and
+ * state back every few iterations and returns when the solve is done, and
  * lbfem_gpu_step_stream, which reads the step's status as lbfem_gpu_step does.
  */
 /* AdvectionOperator::apply (advection.h:49-58, 219-241, 263-289): as lbfem_gpu_advection. */
@@ -442,7 +442,7 @@ int lbfem_gpu_batch_destroy(lbfem_gpu_batch *batch);
  * most 131072 nodes reaches: the most is 2731, Q1 with one cell across.)
  *
  * The call runs eagerly on the context's own stream and is host-synchronous:
- * it reads the solver state back to the host once per CG iteration and
+ * it reads the solver state back to the host every few CG iterations and
  * returns when the solve has finished. It therefore cannot itself be recorded
  * into a CUDA graph. The solve reads x and r on the context's stream, which is
  * not ordered with the caller's streams: the caller must have finished

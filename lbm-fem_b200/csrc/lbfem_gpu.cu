@@ -9,6 +9,7 @@
 #include "contraction_study.cuh"
 #include "quad.cuh"
 #include "batch_group.cuh"
+#include "cg_column.cuh"
 #include "cg_fused.cuh"
 
 #include <cuda_runtime.h>
@@ -683,9 +684,66 @@ namespace
       }
   }
 
+  // Does the solve run on the column kernels (cg_column.cuh)? A product operator of a whole
+  // Cartesian mesh, with the context's own work buffers. From degree 3 on they gain
+  // only on meshes beyond L2: half of a column's x-pass entries are zero there, and
+  // the registers admit fewer threads. FP64 Lee-Lin step, column kernels and element
+  // tiles: 120^2 Q3 409 and 394 us, 60 x 300 Q3 186 and 161, 101 x 77 Q4 461 and 390,
+  // 400^2 Q4 1191 and 1243; against the element tiles with their sums in launches of
+  // their own: 300^2 Q1 113 and 141, 200^2 Q2 380 and 448, 500^2 Q2 1622 and 2106.
+  bool
+  column_solve(const lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c)
+  {
+    if (ctx->strip || c.opk == OPK_LAPLACE || w.state != ctx->d_cg || (ctx->P > 2 && ctx->grid.N < 1000000))
+      return false;
+    for (int s = 0; s < c.nsys; ++s)
+      if (c.opk == OPK_TG3 && !((c.skip >> s) & 1) && c.sc.kxy[s] != 0.)
+        return false;
+    return true;
+  }
+
+  template <int P>
+  dim3
+  col_grid(const Grid &g, int nsys)
+  {
+    const int tw = col_width(g.nfx);
+    return dim3((g.nfx + tw - 1) / tw, (g.nfy + ColShape<P>::RT - 1) / ColShape<P>::RT, nsys);
+  }
+
+  // One phase of a solve on the column kernels: 0 the start, 1 the direction p[1 - pi] from
+  // p[pi], 2 the update with p[pi].
+  int
+  col_launch(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int phase, int pi, const CgFinish &fin)
+  {
+    const Geo geo = geo_of(ctx);
+    return with_degree(ctx->P, [&](auto PP) -> int {
+      constexpr int P = decltype(PP)::value;
+      const dim3 grid = col_grid<P>(ctx->grid, c.nsys);
+      constexpr size_t smem = col_smem<P>();
+      auto go = [&](auto kernel, auto... args) -> cudaError_t {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e == cudaSuccess)
+          kernel<<<grid, ColShape<P>::THREADS, smem, ctx->stream>>>(geo, args...);
+        return e;
+      };
+      auto run = [&](auto SEP) -> cudaError_t {
+        constexpr bool Z = decltype(SEP)::value;
+        if (phase == 0)
+          return go(k_col_start<P, Z>, c.b, c.x_cur, c.x_prev, c.x_new, w.r, c.extrapolate, w.partials, c.sc, c.skip,
+                    w.state, fin);
+        if (phase == 1)
+          return go(k_col_p<P, Z>, w.r, w.p[pi], w.p[1 - pi], w.state, w.partials, c.sc, fin);
+        return go(k_col_update<P, Z>, c.x_new, w.r, w.p[pi], w.state, w.partials, c.sc, fin);
+      };
+      CK((c.opk == OPK_TG3 ? run(std::true_type()) : run(std::false_type())));
+      LAUNCHED();
+      return LBFEM_OK;
+    });
+  }
+
   // r = b - A x_start and the start sums; *n_tiles: the tiles of one system.
   int
-  cg_launch_start(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int *n_tiles)
+  cg_launch_start(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int *n_tiles, const CgFinish &fin)
   {
     const Geo geo = geo_of(ctx);
     return with_degree(ctx->P, [&](auto PP) -> int {
@@ -696,7 +754,7 @@ namespace
       return with_op(c.opk, [&](auto OO) -> int {
         constexpr int OPK = decltype(OO)::value;
         k_cg_start<P, double, double, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(OPK == OPK_MASS ? 0 : 1, true), ctx->stream>>>(
-          geo, c.b, c.x_cur, c.x_prev, c.x_new, w.r, c.extrapolate, w.partials, c.sc, c.skip);
+          geo, c.b, c.x_cur, c.x_prev, c.x_new, w.r, c.extrapolate, w.partials, c.sc, c.skip, w.state, fin);
         LAUNCHED();
         return LBFEM_OK;
       });
@@ -705,7 +763,7 @@ namespace
 
   // p[1-pi] <- D^{-1} r + beta p[pi] and the sums p.Ap.
   int
-  cg_launch_p(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi)
+  cg_launch_p(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi, const CgFinish &fin)
   {
     const Geo geo = geo_of(ctx);
     return with_degree(ctx->P, [&](auto PP) -> int {
@@ -715,7 +773,7 @@ namespace
       return with_op(c.opk, [&](auto OO) -> int {
         constexpr int OPK = decltype(OO)::value;
         k_cg_p<P, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(0), ctx->stream>>>(
-          geo, w.r, w.p[pi], w.p[1 - pi], w.state, w.partials, c.sc);
+          geo, w.r, w.p[pi], w.p[1 - pi], w.state, w.partials, c.sc, fin);
         LAUNCHED();
         return LBFEM_OK;
       });
@@ -724,7 +782,7 @@ namespace
 
   // x += alpha p, r -= alpha A p with p = p[pi], and the sums r.r, r.D^{-1}r.
   int
-  cg_launch_update(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi)
+  cg_launch_update(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi, const CgFinish &fin)
   {
     const Geo geo = geo_of(ctx);
     return with_degree(ctx->P, [&](auto PP) -> int {
@@ -734,7 +792,7 @@ namespace
       return with_op(c.opk, [&](auto OO) -> int {
         constexpr int OPK = decltype(OO)::value;
         k_cg_update<P, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(OPK == OPK_MASS ? 0 : 2), ctx->stream>>>(
-          geo, c.x_new, w.r, w.p[pi], w.state, w.partials, c.sc);
+          geo, c.x_new, w.r, w.p[pi], w.state, w.partials, c.sc, fin);
         LAUNCHED();
         return LBFEM_OK;
       });
@@ -877,6 +935,10 @@ namespace
       }
   }
 
+  // CG iterations launched between two reads of the solver state by the host: a read costs
+  // about 15 us, two kernels that find their systems converged about 5 us.
+  constexpr int CG_AHEAD = 4;
+
   // Jacobi-PCG in the order of updates of deal.II SolverCG (mass.h:204-211),
   // host-driven, with the work buffers w. *its_out: CG iterations summed over
   // the systems.
@@ -907,39 +969,64 @@ namespace
         return cg_status(ctx, ctx->h_cg->status, max_its);
       }
     CK(cudaMemsetAsync(w.state, 0, sizeof(CgState), ctx->stream));
-    if ((st = cg_launch_start(ctx, w, c, &n_tiles)) || (st = reduce_into(ctx, w.partials, w.sums, n_tiles, 3 * NM)) ||
-        (st = strip_allreduce(ctx, 3 * NM)))
+    const bool col = column_solve(ctx, w, c);
+    CgFinish fin;
+    if (!ctx->strip)
+      {
+        fin.nsys = nsys;
+        fin.cg_tol = tol;
+        fin.max_its = max_its;
+      }
+    CgFinish cnt = fin; // the phases after which the host may read the count of active systems
+    cnt.count = 1;
+    // strip mode, the end of a phase: its nq sums, over the ranks, and the scalar work
+    auto phase_end = [&](int phase, int nq) -> int {
+      int s2;
+      if (!ctx->strip)
+        return LBFEM_OK;
+      if ((s2 = reduce_into(ctx, w.partials, w.sums, n_tiles, nq * NM)) || (s2 = strip_allreduce(ctx, nq * NM)))
+        return s2;
+      k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, nsys, phase, tol, max_its);
+      LAUNCHED();
+      return LBFEM_OK;
+    };
+    if (col)
+      st = col_launch(ctx, w, c, 0, 0, cnt);
+    else if (!(st = cg_launch_start(ctx, w, c, &n_tiles, cnt)))
+      st = phase_end(0, 3);
+    if (st || (st = zero_flagged(ctx, c.x_new, w.state, nsys)) || (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
       return st;
-    k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, nsys, 0, tol, max_its);
-    LAUNCHED();
-    if ((st = zero_flagged(ctx, c.x_new, w.state, nsys)) || (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
-      return st;
+    // the state is read back every few iterations (an iteration of converged systems does nothing)
+    const int ahead = ctx->strip || ctx->trace ? 1 : CG_AHEAD;
     int pi = 0;
     for (int it = 0;; ++it)
       {
-        CK(cudaMemcpyAsync(ctx->h_cg, w.state, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (ctx->trace)
+        if (it % ahead == 0)
           {
-            std::fprintf(stderr, "lbfem cg: it %d active %d res/tol", it, ctx->h_cg->n_active);
-            for (int q = 0; q < nsys; ++q)
-              std::fprintf(stderr, " %.2e", ctx->h_cg->tol[q] > 0 ? ctx->h_cg->res[q] / ctx->h_cg->tol[q] : 0.0);
-            std::fprintf(stderr, "\n");
+            CK(cudaMemcpyAsync(ctx->h_cg, w.state, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            if (ctx->trace)
+              {
+                std::fprintf(stderr, "lbfem cg: it %d active %d res/tol", it, ctx->h_cg->n_active);
+                for (int q = 0; q < nsys; ++q)
+                  std::fprintf(stderr, " %.2e", ctx->h_cg->tol[q] > 0 ? ctx->h_cg->res[q] / ctx->h_cg->tol[q] : 0.0);
+                std::fprintf(stderr, "\n");
+              }
+            if (ctx->h_cg->n_active == 0)
+              break;
           }
-        if (ctx->h_cg->n_active == 0)
-          break;
-        if ((st = cg_launch_p(ctx, w, c, pi)) || (st = reduce_into(ctx, w.partials, w.sums, n_tiles, NM)) ||
-            (st = strip_allreduce(ctx, NM)))
+        if (col)
+          {
+            if ((st = col_launch(ctx, w, c, 1, pi, fin)) || (st = col_launch(ctx, w, c, 2, 1 - pi, cnt)))
+              return st;
+            pi = 1 - pi;
+            continue;
+          }
+        if ((st = cg_launch_p(ctx, w, c, pi, fin)) || (st = phase_end(1, 1)))
           return st;
-        k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, nsys, 1, tol, max_its);
-        LAUNCHED();
         pi = 1 - pi;
-        if ((st = cg_launch_update(ctx, w, c, pi)) || (st = reduce_into(ctx, w.partials, w.sums, n_tiles, 2 * NM)) ||
-            (st = strip_allreduce(ctx, 2 * NM)))
-          return st;
-        k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, nsys, 2, tol, max_its);
-        LAUNCHED();
-        if ((st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
+        if ((st = cg_launch_update(ctx, w, c, pi, cnt)) || (st = phase_end(2, 2)) ||
+            (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
           return st;
       }
     if (its_out)
@@ -1082,7 +1169,7 @@ namespace
               n_tiles = int(grid.x * grid.y);
               grid.z = nsys;
               k_cg_start<P, float, float, double><<<grid, THREADS, cg_smem<P, float>(1, true), ctx->stream>>>(
-                geo, b, nullptr, nullptr, xs, r_in, 0, ctx->d_partials, StreamCoef{}, 0);
+                geo, b, nullptr, nullptr, xs, r_in, 0, ctx->d_partials, StreamCoef{}, 0, nullptr, CgFinish{});
               LAUNCHED();
               return LBFEM_OK;
             });
@@ -1800,36 +1887,32 @@ namespace
     cudaGraphConditionalHandle h;
     CK(cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault)); // 0 at every launch
     CK(cudaMemsetAsync(w.state, 0, sizeof(CgState), ctx->stream));
+    CgFinish fin, set; // set: also sets the loop's condition
+    fin.nsys = c.nsys;
+    fin.cg_tol = tol;
+    fin.max_its = max_its;
+    set = fin;
+    set.count = 1;
+    set.ds = ctx->d_stats;
+    set.h = h;
+    const bool col = column_solve(ctx, w, c);
     int n_tiles = 0, st;
-    if ((st = cg_launch_start(ctx, w, c, &n_tiles)) || (st = reduce_into(ctx, w.partials, w.sums, n_tiles, 3 * NM)))
+    if ((st = col ? col_launch(ctx, w, c, 0, 0, set) : cg_launch_start(ctx, w, c, &n_tiles, set)) ||
+        (st = zero_flagged(ctx, c.x_new, w.state, c.nsys)))
       return st;
-    k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, c.nsys, 0, tol, max_its);
-    LAUNCHED();
-    if ((st = zero_flagged(ctx, c.x_new, w.state, c.nsys)))
-      return st;
-    k_cg_control<<<1, 32, 0, ctx->stream>>>(w.state, ctx->d_stats, h, 0);
-    LAUNCHED();
-    auto iteration = [&](int pi) -> int {
+    auto iteration = [&](int pi, const CgFinish &end) -> int {
       int s2;
-      if ((s2 = cg_launch_p(ctx, w, c, pi)) || (s2 = reduce_into(ctx, w.partials, w.sums, n_tiles, NM)))
-        return s2;
-      k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, c.nsys, 1, tol, max_its);
-      LAUNCHED();
-      if ((s2 = cg_launch_update(ctx, w, c, 1 - pi)) || (s2 = reduce_into(ctx, w.partials, w.sums, n_tiles, 2 * NM)))
-        return s2;
-      k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, c.nsys, 2, tol, max_its);
-      LAUNCHED();
-      return LBFEM_OK;
+      if (col)
+        (s2 = col_launch(ctx, w, c, 1, pi, fin)) || (s2 = col_launch(ctx, w, c, 2, 1 - pi, end));
+      else
+        (s2 = cg_launch_p(ctx, w, c, pi, fin)) || (s2 = cg_launch_update(ctx, w, c, 1 - pi, end));
+      return s2;
     };
     return capture_while(
       ctx, h,
       [&]() -> int {
-        int s2;
-        if ((s2 = iteration(0)) || (s2 = iteration(1)))
-          return s2;
-        k_cg_control<<<1, 32, 0, ctx->stream>>>(w.state, ctx->d_stats, h, 1);
-        LAUNCHED();
-        return LBFEM_OK;
+        const int s2 = iteration(0, fin);
+        return s2 ? s2 : iteration(1, set);
       },
       body_kernels);
   }
@@ -2545,8 +2628,8 @@ lbfem_gpu_create(const lbfem_mesh_desc *m, const lbfem_params *prm, lbfem_gpu_ct
     }
   const long long tiles = with_degree(P, [&](auto PP) -> int {
     constexpr int Pd = decltype(PP)::value;
-    const dim3 tg = tile_grid<Pd>(ctx->grid);
-    return int(tg.x * tg.y);
+    const dim3 tg = tile_grid<Pd>(ctx->grid), cg = col_grid<Pd>(ctx->grid, 1);
+    return int(std::max(tg.x * tg.y, cg.x * cg.y));
   });
   ctx->partial_cap = size_t(std::max<long long>(tiles, 148 * 8)) * 3 * NM;
   if ((st = zeros(&ctx->d_partials, ctx->partial_cap)) || (st = zeros(&ctx->d_sums, 64)))

@@ -1527,8 +1527,210 @@ namespace lbfem_gpu
     int it[NM], its_total[NM], active[NM];
     int zero[NM]; // the system's right-hand side is exactly zero: its solution is 0 (k_zero_flagged)
     int status, n_active, iter;
+    int ticket[NM], systems_done; // CTAs of a system, systems that have finished a phase (cg_finish)
     unsigned long long total_its;
   };
+
+  // What the scalar work of a phase reads of system s, fetched at once and ahead of the sums.
+  struct CgSystem
+  {
+    int active, it, its_total, status;
+    double tol, rz;
+  };
+
+  __device__ __forceinline__ CgSystem
+  cg_system(const CgState *st, int s)
+  {
+    return {st->active[s], st->it[s], st->its_total[s], st->status, st->tol[s], st->rz[s]};
+  }
+
+  // The scalar work of one CG phase for system s (state q). phase 0 (after the start): v = b.b,
+  // r.r, r.D^{-1}r; phase 1 (after p): p.Ap; phase 2 (after the update): r.r, r.D^{-1}r.
+  __device__ __forceinline__ void
+  cg_scalars(CgState *st, int s, const CgSystem &q, const double *v, int phase, double cg_tol, int max_its)
+  {
+    if (phase == 0)
+      {
+        if (q.status != 0 || q.its_total >= max_its)
+          {
+            st->active[s] = 0;
+            return;
+          }
+        const double tol = cg_tol * sqrt(v[0]), res = sqrt(v[1]);
+        const bool zero = v[0] == 0.0;
+        st->tol[s] = tol;
+        st->res[s] = res;
+        st->rz[s] = v[2];
+        st->it[s] = 0;
+        st->beta[s] = 0;
+        st->zero[s] = zero;
+        st->active[s] = isnan(res) || res <= tol || zero ? 0 : 1;
+        if (isnan(res))
+          atomicExch(&st->status, 3); // LBFEM_ERR_NONFINITE
+      }
+    else if (!q.active)
+      return;
+    else if (phase == 1)
+      st->alpha[s] = q.rz / v[0];
+    else
+      {
+        const int it = q.its_total + 1;
+        st->it[s] = q.it + 1;
+        st->its_total[s] = it;
+        atomicAdd(&st->total_its, 1ULL);
+        const double res = sqrt(v[0]);
+        st->res[s] = res;
+        if (isnan(res))
+          {
+            st->active[s] = 0;
+            atomicExch(&st->status, 3);
+          }
+        else if (res <= q.tol)
+          st->active[s] = 0;
+        else if (it >= max_its)
+          {
+            st->active[s] = 0;
+            atomicCAS(&st->status, 0, 2); // LBFEM_ERR_NO_CONVERGENCE
+          }
+        else
+          {
+            st->rz_prev[s] = q.rz;
+            st->rz[s] = v[1];
+            st->beta[s] = v[1] / q.rz;
+          }
+      }
+  }
+
+  // The count of active systems after a phase of all of them.
+  __device__ __forceinline__ void
+  cg_count(CgState *st, int phase)
+  {
+    volatile CgState *vs = st; // other CTAs wrote them
+    int n = 0;
+    for (int k = 0; k < NM; ++k)
+      n += vs->active[k];
+    st->n_active = n;
+    if (phase == 2)
+      ++st->iter;
+  }
+
+  // Graph control after a CG phase: the loop goes on while a system is active and no
+  // failure occurred; on exit the solve is folded into the counters.
+  __device__ __forceinline__ void
+  cg_control(const CgState *st, DevStats *ds, cudaGraphConditionalHandle h, bool in_body)
+  {
+    volatile const CgState *vs = st;
+    const int status = vs->status;
+    const bool go = vs->n_active > 0 && status == 0;
+    if (in_body)
+      ++ds->bodies;
+    if (!go)
+      {
+        ds->its += vs->total_its;
+        if (status != 0 && ds->sticky == 0)
+          ds->sticky = status;
+      }
+    cudaGraphSetConditional(h, go ? 1u : 0u);
+  }
+
+  // The rest of a CG phase that its kernel does in its last CTAs (cg_finish); nsys 0: nothing,
+  // the sums are reduced, and added over the ranks of a decomposed mesh, by other launches.
+  struct CgFinish
+  {
+    int nsys = 0;
+    double cg_tol = 0;
+    int max_its = 0;
+    int count = 0;                    // count the active systems (and with ds set the loop's condition)
+    DevStats *ds = nullptr;           // set with h: the last phase of a loop body (or the start)
+    cudaGraphConditionalHandle h = 0; // sets the loop's condition
+  };
+
+  // System s is done with a phase (one thread of its last CTA): the last system to finish
+  // counts the active ones and sets the loop's condition, where something reads them.
+  __device__ __forceinline__ void
+  cg_system_done(CgState *st, const CgFinish &fin, int phase)
+  {
+    if (!fin.count)
+      return;
+    __threadfence();
+    if (atomicAdd(&st->systems_done, 1) != fin.nsys - 1)
+      return;
+    __threadfence();
+    st->systems_done = 0;
+    cg_count(st, phase);
+    if (fin.ds)
+      cg_control(st, fin.ds, fin.h, phase != 0);
+  }
+
+  // The last CTA of system s: the sums of the partial sums in a fixed order, and the phase's
+  // scalar work. Not inlined: its registers would spill the kernels that end with it.
+  template <int NQ, int NT>
+  __device__ __noinline__ void
+  cg_last_cta(const double *__restrict__ partials, CgState *st, int s, int nt, int phase, const CgFinish *fin)
+  {
+    __shared__ double red[NQ][NT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __threadfence();
+    CgSystem sys{};
+    if (threadIdx.x == 0)
+      sys = cg_system(st, s);
+    double v[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      v[q] = 0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nt; b += NT)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        v[q] += __ldcg(partials + (long long)(q * NM + s) * nt + b);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+        if (lane == 0)
+          red[q][warp] = v[q];
+      }
+    __syncthreads();
+    if (threadIdx.x != 0)
+      return;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      {
+        v[q] = red[q][0];
+        for (int w = 1; w < NT / 32; ++w)
+          v[q] += red[q][w];
+      }
+    st->ticket[s] = 0;
+    const double sums[3] = {v[0], NQ > 1 ? v[1 % NQ] : 0., NQ > 2 ? v[2 % NQ] : 0.};
+    cg_scalars(st, s, sys, sums, phase, fin->cg_tol, fin->max_its);
+    cg_system_done(st, *fin, phase);
+  }
+
+  // The end of a CG kernel's tile `tile` of nt for system s: its partial sums stored; the
+  // system's last CTA to arrive adds them and does the phase's scalar work. A sums kernel
+  // and a scalar kernel instead cost about 5 us a phase; this costs 2 to 3, the chain of
+  // fences and L2 round trips from the last store to the new scalars (101 x 77 Q4: 431 to
+  // 390 us per step at 8 iterations).
+  template <int NQ, int NT>
+  __device__ __forceinline__ void
+  cg_finish(double (&part)[NQ], double *__restrict__ partials, CgState *st, int s, int tile, int nt, int phase,
+            const CgFinish &fin)
+  {
+    block_reduce_store_n<NQ, NT>(part, partials + (long long)s * nt, tile, NM * nt);
+    if (!fin.nsys)
+      return;
+    __shared__ int last;
+    if (threadIdx.x == 0)
+      {
+        __threadfence(); // this thread stored the CTA's sums
+        last = atomicAdd(&st->ticket[s], 1) == nt - 1;
+      }
+    __syncthreads();
+    if (last)
+      cg_last_cta<NQ, NT>(partials, st, s, nt, phase, &fin);
+  }
 
   // x_s <- 0 for the systems whose right-hand side is exactly zero. deal.II's
   // SolverCG would iterate from a nonzero (extrapolated) start toward the
@@ -1588,7 +1790,8 @@ namespace lbfem_gpu
   __device__ __forceinline__ void
   cg_start_tile(const Geo &geo, const R *__restrict__ b, const X *__restrict__ x_cur, const X *__restrict__ x_prev,
                 X *__restrict__ x_new, R *__restrict__ r, int extrapolate, double *__restrict__ partials,
-                const StreamCoef &sc, int skip, int bx, int by, int bz, int nbx, int nby)
+                const StreamCoef &sc, int skip, int bx, int by, int bz, int nbx, int nby, CgState *st,
+                const CgFinish &fin)
   {
     using T = Tile<P>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -1605,6 +1808,12 @@ namespace lbfem_gpu
             const int nt = nbx * nby, tile = by * nbx + bx;
             for (int q = 0; q < 3; ++q)
               partials[(long long)(q * NM + s) * nt + tile] = 0.0;
+            if (fin.nsys && tile == 0)
+              {
+                const double v[3] = {0., 0., 0.};
+                cg_scalars(st, s, cg_system(st, s), v, 0, fin.cg_tol, fin.max_its);
+                cg_system_done(st, fin, 0);
+              }
           }
         return;
       }
@@ -1652,9 +1861,8 @@ namespace lbfem_gpu
     });
     if constexpr (SUMS)
       {
-        const int nt = nbx * nby, tile = by * nbx + bx;
         // partial (quantity k of system s) at [(k*NM + s) * n_tiles + tile]
-        block_reduce_store<3>(part, partials + (long long)s * nt, tile, NM * nt);
+        cg_finish<3, THREADS>(part, partials, st, s, by * nbx + bx, nbx * nby, 0, fin);
       }
   }
 
@@ -1662,17 +1870,17 @@ namespace lbfem_gpu
   __global__ void __launch_bounds__(THREADS, OPK != OPK_MASS ? 2 : sizeof(R) == sizeof(float) ? 8 : 6)
     k_cg_start(const Geo geo, const R *__restrict__ b, const X *__restrict__ x_cur, const X *__restrict__ x_prev,
                X *__restrict__ x_new, R *__restrict__ r, int extrapolate, double *__restrict__ partials,
-               const StreamCoef sc, int skip)
+               const StreamCoef sc, int skip, CgState *st, const CgFinish fin)
   {
     cg_start_tile<P, R, X, A, OPK>(geo, b, x_cur, x_prev, x_new, r, extrapolate, partials, sc, skip, blockIdx.x,
-                                   blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
+                                   blockIdx.y, blockIdx.z, gridDim.x, gridDim.y, st, fin);
   }
 
   // p <- D^{-1} r + beta p (p <- D^{-1} r on the first iteration); partial p.Ap. One system per CTA.
   template <int P, typename R, int OPK = OPK_MASS>
   __global__ void __launch_bounds__(THREADS, OPK == OPK_MASS ? 8 : 2)
     k_cg_p(const Geo geo, const R *__restrict__ r, const R *__restrict__ p_in, R *__restrict__ p_out,
-           const CgState *__restrict__ st, double *__restrict__ partials, const StreamCoef sc)
+           CgState *st, double *__restrict__ partials, const StreamCoef sc, const CgFinish fin)
   {
     using T = Tile<P>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -1683,7 +1891,11 @@ namespace lbfem_gpu
     const int s = blockIdx.z;
     const int nt = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
     if (!st->active[s])
-      return;
+      {
+        if (fin.nsys && tile == 0 && threadIdx.x == 0)
+          cg_system_done(st, fin, 1);
+        return;
+      }
     const int gx0 = blockIdx.x * T::TX, gy0 = blockIdx.y * T::TY;
     build_maps<P>(maps, geo, gx0, gy0);
     const bool first = st->it[s] == 0;
@@ -1712,14 +1924,14 @@ namespace lbfem_gpu
       if (owned_row(gy0 + i, g))
         part[0] += double(pn) * double(Ap);
     });
-    block_reduce_store<1>(part, partials + (long long)s * nt, tile, NM * nt);
+    cg_finish<1, THREADS>(part, partials, st, s, tile, nt, 1, fin);
   }
 
   // v = A p recomputed; x += alpha p, r -= alpha v; partials r.r, r.D^{-1}r. One system per CTA.
   template <int P, typename R, int OPK = OPK_MASS>
   __global__ void __launch_bounds__(THREADS, OPK == OPK_MASS ? 8 : 2)
     k_cg_update(const Geo geo, R *__restrict__ x, R *__restrict__ r, const R *__restrict__ p,
-                const CgState *__restrict__ st, double *__restrict__ partials, const StreamCoef sc)
+                CgState *st, double *__restrict__ partials, const StreamCoef sc, const CgFinish fin)
   {
     using T = Tile<P>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -1730,7 +1942,11 @@ namespace lbfem_gpu
     const int s = blockIdx.z;
     const int nt = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
     if (!st->active[s])
-      return;
+      {
+        if (fin.nsys && tile == 0 && threadIdx.x == 0)
+          cg_system_done(st, fin, 2);
+        return;
+      }
     const int gx0 = blockIdx.x * T::TX, gy0 = blockIdx.y * T::TY;
     build_maps<P>(maps, geo, gx0, gy0);
     const R al = R(st->alpha[s]);
@@ -1765,7 +1981,7 @@ namespace lbfem_gpu
           part[1] += double(rr) * (cg_inv_jacobi<P, OPK>(geo, maps, gx0, gy0, i, j, image) * double(rr));
         }
     });
-    block_reduce_store<2>(part, partials + (long long)s * nt, tile, NM * nt);
+    cg_finish<2, THREADS>(part, partials, st, s, tile, nt, 2, fin);
   }
 
   // --------------------------- tensor-product window solve (mixed precision)
@@ -2397,101 +2613,23 @@ namespace lbfem_gpu
                            blockIdx.z, gridDim.x, gridDim.y);
   }
 
-  // The scalar work of one CG phase, one thread per system, from the reduced sums.
-  // phase 0 (after start): sums = [bb, rr, rz]; phase 1 (after p): [pAp];
-  // phase 2 (after update): [rr, rz].
+  // The scalar work of one CG phase, one thread per system, from the reduced sums
+  // (sums[q * NM + s]), for a decomposed mesh.
   __global__ void
   k_cg_scalars(CgState *st, const double *__restrict__ sums, int nsys, int phase, double cg_tol, int max_its)
   {
     const int s = threadIdx.x;
-    if (s < NM)
+    if (s < nsys)
       {
-        if (phase == 0)
-          {
-            if (s < nsys && st->status == 0 && st->its_total[s] < max_its)
-              {
-                st->tol[s] = cg_tol * sqrt(sums[s]);
-                const double res = sqrt(sums[NM + s]);
-                st->res[s] = res;
-                st->rz[s] = sums[2 * NM + s];
-                st->it[s] = 0;
-                st->beta[s] = 0;
-                st->zero[s] = sums[s] == 0.0;
-                if (isnan(res))
-                  {
-                    st->active[s] = 0;
-                    atomicExch(&st->status, 3); // LBFEM_ERR_NONFINITE
-                  }
-                else
-                  st->active[s] = (res <= st->tol[s] || st->zero[s]) ? 0 : 1;
-              }
-            else
-              st->active[s] = 0;
-          }
-        else if (phase == 1)
-          {
-            if (s < nsys && st->active[s])
-              st->alpha[s] = st->rz[s] / sums[s];
-          }
-        else if (s < nsys && st->active[s])
-          {
-            ++st->it[s];
-            const int it = ++st->its_total[s];
-            atomicAdd(&st->total_its, 1ULL);
-            const double res = sqrt(sums[s]);
-            st->res[s] = res;
-            if (isnan(res))
-              {
-                st->active[s] = 0;
-                atomicExch(&st->status, 3);
-              }
-            else if (res <= st->tol[s])
-              st->active[s] = 0;
-            else if (it >= max_its)
-              {
-                st->active[s] = 0;
-                atomicCAS(&st->status, 0, 2); // LBFEM_ERR_NO_CONVERGENCE
-              }
-            else
-              {
-                st->rz_prev[s] = st->rz[s];
-                st->rz[s] = sums[NM + s];
-                st->beta[s] = st->rz[s] / st->rz_prev[s];
-              }
-          }
+        const double v[3] = {sums[s], phase == 1 ? 0. : sums[NM + s], phase == 0 ? sums[2 * NM + s] : 0.};
+        cg_scalars(st, s, cg_system(st, s), v, phase, cg_tol, max_its);
       }
     __syncthreads();
     if (threadIdx.x == 0)
-      {
-        int n = 0;
-        for (int k = 0; k < NM; ++k)
-          n += st->active[k];
-        st->n_active = n;
-        if (phase == 2)
-          ++st->iter;
-      }
+      cg_count(st, phase);
   }
 
   // ------------------------------------------------- device-side step control
-  // Graph control after a CG phase: the loop goes on while a system is active
-  // and no failure occurred; on exit the solve is folded into the counters.
-  __global__ void
-  k_cg_control(const CgState *__restrict__ st, DevStats *__restrict__ ds, cudaGraphConditionalHandle h, int in_body)
-  {
-    if (threadIdx.x != 0)
-      return;
-    const bool go = st->n_active > 0 && st->status == 0;
-    if (in_body)
-      ++ds->bodies;
-    if (!go)
-      {
-        ds->its += st->total_its;
-        if (st->status != 0 && ds->sticky == 0)
-          ds->sticky = st->status;
-      }
-    cudaGraphSetConditional(h, go ? 1u : 0u);
-  }
-
   // The bookkeeping of one round of the mixed-precision mass solve, after the
   // round's correction kernel and the reduction of its sums [bb, rr]: a
   // corrected system whose residual meets tol stops; a round that halves no
