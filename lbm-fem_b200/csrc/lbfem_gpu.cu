@@ -1487,10 +1487,6 @@ namespace
     return launch_wall_faces<double>(ctx, bardow ? g : f, ctx->d_rhs, e, dt, remove);
   }
 
-  // The nodal update of sweep s with its increment (x_cur, or d_x[s] for a split
-  // sweep). Bardow: f = g* + x (TaylorGalerkin::stream, streaming.h:88-100),
-  // which flips the population buffers after the last sweep; Lee-Lin: the
-  // predictor-corrector.
   // With the lumped mass (of a whole mesh) the update solves for its increment itself.
   bool
   lumped_update(const lbfem_gpu_ctx *ctx)
@@ -1498,6 +1494,10 @@ namespace
     return ctx->prm.mass == LBFEM_MASS_LUMPED && !ctx->strip && !ctx->distorted;
   }
 
+  // The nodal update of sweep s with its increment (x_cur, or d_x[s] for a split
+  // sweep). Bardow: f = g* + x (TaylorGalerkin::stream, streaming.h:88-100),
+  // which flips the population buffers after the last sweep; Lee-Lin: the
+  // predictor-corrector.
   int
   step_back(lbfem_gpu_ctx *ctx, int sweep = 0)
   {
