@@ -810,6 +810,11 @@ namespace
   }
 
   // ------------------------------------------------ the solve in one launch
+  // The most dynamic shared memory a CTA of k_cg_fused asks for. The kernel's limit is set to it
+  // before every launch, whatever the mesh needs: the limit belongs to the process, and one
+  // host thread's smaller limit would refuse another's launch or step graph.
+  constexpr size_t FUSED_SMEM = 200 * 1024;
+
   // How k_cg_fused runs a solve of this context, if it does (group > 0): one cluster of
   // `group` CTAs per system.
   struct FusedPlan
@@ -855,7 +860,7 @@ namespace
           const int ncr = (g.ncy + group - 1) / group; // the most cell rows of a band, the last one included
           const size_t bytes = sizeof(double) * size_t(fused_smem_doubles<P>(g.nfx, g.ncx, ncr));
           const long long tasks = (long long)(ncr + 1) * g.nfx;
-          if (group > g.ncy || bytes > size_t(group == 8 ? 200 : 100) * 1024 || tasks > (long long)S::MAXT * most)
+          if (group > g.ncy || bytes > (group == 8 ? FUSED_SMEM : FUSED_SMEM / 2) || tasks > (long long)S::MAXT * most)
             continue;
           f.group = group;
           f.threads = int(std::min<long long>(most, (tasks + 31) / 32 * 32));
@@ -873,7 +878,7 @@ namespace
   {
     // set here and not when a context is made: only the solves of small meshes load the kernel
     auto kernel = k_cg_fused<P, SEP>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(f.smem));
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FUSED_SMEM));
     if (e == cudaSuccess && f.group > 8)
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess)
