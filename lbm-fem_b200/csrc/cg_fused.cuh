@@ -478,13 +478,17 @@ namespace lbfem_gpu
         st->zero[s] = zero ? 1 : 0;
         st->active[s] = 0;
         atomicAdd(&st->total_its, (unsigned long long)it);
-        if (A.ds)
-          atomicAdd(&A.ds->its, (unsigned long long)it);
+        // a non-finite system (3) wins over the iteration cap (2), whichever ends first
         if (status)
+          atomicMax(&st->status, status);
+        if (A.ds)
           {
-            atomicCAS(&st->status, 0, status);
-            if (A.ds)
-              atomicCAS(&A.ds->sticky, 0, status);
+            __threadfence();
+            if (atomicAdd(&st->systems_done, 1) == int(gridDim.x) / group - 1)
+              {
+                __threadfence();
+                cg_fold(st, A.ds);
+              }
           }
       }
   }

@@ -1657,22 +1657,28 @@ namespace lbfem_gpu
       ++st->iter;
   }
 
+  // A finished solve folded into the counters: its iterations, and its status if it failed.
+  __device__ __forceinline__ void
+  cg_fold(const CgState *st, DevStats *ds)
+  {
+    volatile const CgState *vs = st; // other CTAs wrote them
+    const int status = vs->status;
+    ds->its += vs->total_its;
+    if (status != 0 && ds->sticky == 0)
+      ds->sticky = status;
+  }
+
   // Graph control after a CG phase: the loop goes on while a system is active and no
   // failure occurred; on exit the solve is folded into the counters.
   __device__ __forceinline__ void
   cg_control(const CgState *st, DevStats *ds, cudaGraphConditionalHandle h, bool in_body)
   {
     volatile const CgState *vs = st;
-    const int status = vs->status;
-    const bool go = vs->n_active > 0 && status == 0;
+    const bool go = vs->n_active > 0 && vs->status == 0;
     if (in_body)
       ++ds->bodies;
     if (!go)
-      {
-        ds->its += vs->total_its;
-        if (status != 0 && ds->sticky == 0)
-          ds->sticky = status;
-      }
+      cg_fold(st, ds);
     cudaGraphSetConditional(h, go ? 1u : 0u);
   }
 
