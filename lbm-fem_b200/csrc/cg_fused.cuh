@@ -38,7 +38,7 @@ namespace lbfem_gpu
     DevStats *ds;     // counters of a graph-launched step, or null
     StreamCoef sc;
     int sys[NM];      // the systems solved, in cluster order
-    int extrapolate, group; // group: CTAs per cluster
+    int extrapolate;
     double cg_tol;
     int max_its;
   };
@@ -50,7 +50,7 @@ namespace lbfem_gpu
   struct FusedShape
   {
     static constexpr int THREADS = 512; // most threads of a CTA
-    static constexpr int GROUP = 16;    // most CTAs of a cluster
+    static constexpr int GROUP = 8;     // CTAs of a cluster: the largest portable size
     static constexpr int MAXT = P == 1 ? 10 : P == 2 ? 5 : P == 3 ? 4 : 2;
   };
 
@@ -126,7 +126,8 @@ namespace lbfem_gpu
     __shared__ double s_slot[4][S::GROUP * MW]; // the warps' partial sums of all CTAs of the cluster
     const Grid &g = geo.g;
     const int nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt / 32;
-    const int group = A.group, s = A.sys[blockIdx.x / group], rank = blockIdx.x % group;
+    constexpr int group = S::GROUP;
+    const int s = A.sys[blockIdx.x / group], rank = blockIdx.x % group;
     const int nfx = g.nfx, ncx = g.ncx, pitch = nfx | 1;
     int c0, c1;
     fused_band(g.ncy, group, rank, c0, c1);

@@ -815,25 +815,25 @@ namespace
   // host thread's smaller limit would refuse another's launch or step graph.
   constexpr size_t FUSED_SMEM = 200 * 1024;
 
-  // How k_cg_fused runs a solve of this context, if it does (group > 0): one cluster of
-  // `group` CTAs per system.
+  // How k_cg_fused runs a solve of this context, if it does (n > 0): one cluster per system.
   struct FusedPlan
   {
-    int group = 0, threads = 0;
+    int threads = 0;
     size_t smem = 0;
     int n = 0, sys[NM] = {};
     bool sep = false;
   };
 
   // The solve runs in one launch when its operator is a product (the mass matrix, or the
-  // TG3 matrix of axis-parallel directions) and a system fits in a cluster: its
-  // shared memory, and a thread's share of the nodes in its registers. Clusters of 8
-  // CTAs of up to 512 threads, one CTA per SM, of which 15 are resident at once; else
-  // of 16 CTAs of up to 256 threads, which must fit an SM in pairs (7 clusters of 16
-  // are resident with one CTA per SM, 14 with two). Measured per step, FP64 Bardow at
-  // tolerance 1e-10, clusters of 8 / of 16 / the loop of kernels: 64^2 Q1 85 / 89 /
-  // 226 us, 180^2 Q1 105 / 109 / 193 us, 64^2 Q2 162 / 177 / 458 us, 32^2 Q4 157 /
-  // 168 / 450 us.
+  // TG3 matrix of axis-parallel directions) and a system fits in a cluster of 8 CTAs of up to
+  // 512 threads: its shared memory, and a thread's share of the nodes in its registers
+  // (196^2 Q1, 193^2 Q2, 202^2 Q3 or 161^2 Q4 nodes on square meshes). One CTA per SM, of which
+  // 15 clusters are resident at once. Measured per step, FP64 Bardow at tolerance 1e-10, one
+  // launch / the loop of kernels: 64^2 Q1 85 / 226 us, 180^2 Q1 105 / 193 us, 64^2 Q2
+  // 162 / 458 us, 32^2 Q4 157 / 450 us. Clusters of 16 CTAs of half the threads and
+  // shared memory (two CTAs per SM) admit no mesh that 8 do not, and took 4 to 9% longer.
+  // The blocks of skipped systems are not touched: they have to be zero already, as a split
+  // sweep's are (its x starts at zero and nothing else writes the resting populations').
   FusedPlan
   fused_plan(const lbfem_gpu_ctx *ctx, const CgCall &c)
   {
@@ -842,33 +842,21 @@ namespace
       return f;
     f.sep = c.opk == OPK_TG3;
     for (int s = 0; s < c.nsys; ++s)
-      if (!((c.skip >> s) & 1))
-        {
-          if (f.sep && c.sc.kxy[s] != 0.)
-            return f;
-          f.sys[f.n++] = s;
-        }
-    if (f.n == 0)
-      return f;
+      if (f.sep && !((c.skip >> s) & 1) && c.sc.kxy[s] != 0.)
+        return f;
     const Grid &g = ctx->grid;
-    with_degree(ctx->P, [&](auto PP) -> int {
+    const bool fits = with_degree(ctx->P, [&](auto PP) -> int {
       constexpr int P = decltype(PP)::value;
       using S = FusedShape<P>;
-      for (const int group : {8, 16})
-        {
-          const int most = group == 8 ? S::THREADS : S::THREADS / 2;
-          const int ncr = (g.ncy + group - 1) / group; // the most cell rows of a band, the last one included
-          const size_t bytes = sizeof(double) * size_t(fused_smem_doubles<P>(g.nfx, g.ncx, ncr));
-          const long long tasks = (long long)(ncr + 1) * g.nfx;
-          if (group > g.ncy || bytes > (group == 8 ? FUSED_SMEM : FUSED_SMEM / 2) || tasks > (long long)S::MAXT * most)
-            continue;
-          f.group = group;
-          f.threads = int(std::min<long long>(most, (tasks + 31) / 32 * 32));
-          f.smem = bytes;
-          break;
-        }
-      return 0;
+      const int ncr = (g.ncy + S::GROUP - 1) / S::GROUP; // the most cell rows of a band, the last one included
+      f.smem = sizeof(double) * size_t(fused_smem_doubles<P>(g.nfx, g.ncx, ncr));
+      const long long tasks = (long long)(ncr + 1) * g.nfx;
+      f.threads = int(std::min<long long>(S::THREADS, (tasks + 31) / 32 * 32));
+      return S::GROUP <= g.ncy && f.smem <= FUSED_SMEM && tasks <= (long long)S::MAXT * S::THREADS;
     });
+    for (int s = 0; s < c.nsys && fits; ++s)
+      if (!((c.skip >> s) & 1))
+        f.sys[f.n++] = s;
     return f;
   }
 
@@ -878,19 +866,17 @@ namespace
   {
     // set here and not when a context is made: only the solves of small meshes load the kernel
     auto kernel = k_cg_fused<P, SEP>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FUSED_SMEM));
-    if (e == cudaSuccess && f.group > 8)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FUSED_SMEM));
     if (e != cudaSuccess)
       return e;
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(f.group * f.n);
+    lc.gridDim = dim3(FusedShape<P>::GROUP * f.n);
     lc.blockDim = dim3(f.threads);
     lc.dynamicSmemBytes = f.smem;
     lc.stream = stream;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = f.group;
+    at.val.clusterDim.x = FusedShape<P>::GROUP;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     lc.attrs = &at;
     lc.numAttrs = 1;
@@ -912,7 +898,6 @@ namespace
     for (int k = 0; k < f.n; ++k)
       a.sys[k] = f.sys[k];
     a.extrapolate = c.extrapolate;
-    a.group = f.group;
     a.cg_tol = c.tol >= 0 ? c.tol : ctx->prm.cg_tolerance;
     a.max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
     const Geo geo = geo_of(ctx);
@@ -955,7 +940,7 @@ namespace
     const int nsys = c.nsys;
     int n_tiles = 0, st;
     const FusedPlan f = w.state == ctx->d_cg ? fused_plan(ctx, c) : FusedPlan{};
-    if (f.group)
+    if (f.n)
       {
         if ((st = fused_solve(ctx, f, w.state, c, nullptr)))
           return st;
@@ -1901,7 +1886,7 @@ namespace
     const int max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
     const CgScratch<double> w = ctx_scratch(ctx);
     const FusedPlan f = fused_plan(ctx, c);
-    if (f.group)
+    if (f.n)
       {
         *body_kernels = 0;
         return fused_solve(ctx, f, w.state, c, ctx->d_stats);
