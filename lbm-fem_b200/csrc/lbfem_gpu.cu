@@ -70,6 +70,7 @@ struct lbfem_gpu_ctx
   size_t partial_cap = 0;
   CgState *d_cg = nullptr;
   CgState *h_cg = nullptr; // pinned mirror
+  int fused_ok[2] = {-1, -1}; // can the one-launch solve's clusters be resident (mass, TG3)? -1: not asked yet
   double dt = 0, lambda = 0;
   bool have_ts = false;
   int64_t cg_its = 0;
@@ -811,8 +812,8 @@ namespace
 
   // ------------------------------------------------ the solve in one launch
   // The most dynamic shared memory a CTA of k_cg_fused asks for. The kernel's limit is set to it
-  // before every launch, whatever the mesh needs: the limit belongs to the process, and one
-  // host thread's smaller limit would refuse another's launch or step graph.
+  // whatever the mesh needs: the limit belongs to the process, and one host thread's smaller
+  // limit would refuse another's launch or step graph.
   constexpr size_t FUSED_SMEM = 200 * 1024;
 
   // How k_cg_fused runs a solve of this context, if it does (n > 0): one cluster per system.
@@ -823,6 +824,54 @@ namespace
     int n = 0, sys[NM] = {};
     bool sep = false;
   };
+
+  // The launch of n clusters of plan f; at: the storage of its attribute.
+  cudaLaunchConfig_t
+  fused_config(const FusedPlan &f, int n, int group, cudaLaunchAttribute *at, cudaStream_t stream)
+  {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(group * n);
+    lc.blockDim = dim3(f.threads);
+    lc.dynamicSmemBytes = f.smem;
+    lc.stream = stream;
+    *at = {};
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = group;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return lc;
+  }
+
+  // Can a cluster of plan f be resident? Not on a partition of the device with too few
+  // SMs beside each other: the solve then takes the loop of kernels. Asked once per context
+  // and operator (f's threads and shared memory follow from the mesh), with the kernel's
+  // shared-memory limit set first; not when a context is made, since only the solves of small
+  // meshes load the kernel.
+  bool
+  fused_resident(lbfem_gpu_ctx *ctx, const FusedPlan &f)
+  {
+    int &ok = ctx->fused_ok[f.sep];
+    if (ok >= 0)
+      return ok;
+    ok = with_degree(ctx->P, [&](auto PP) -> int {
+      constexpr int P = decltype(PP)::value;
+      auto ask = [&](auto kernel) -> int {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t lc = fused_config(f, 1, FusedShape<P>::GROUP, &at, nullptr);
+        int n = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FUSED_SMEM)) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess)
+          {
+            cudaGetLastError(); // the answer is no
+            n = 0;
+          }
+        return n > 0;
+      };
+      return f.sep ? ask(k_cg_fused<P, true>) : ask(k_cg_fused<P, false>);
+    });
+    return ok;
+  }
 
   // The solve runs in one launch when its operator is a product (the mass matrix, or the
   // TG3 matrix of axis-parallel directions) and a system fits in a cluster of 8 CTAs of up to
@@ -835,7 +884,7 @@ namespace
   // The blocks of skipped systems are not touched: they have to be zero already, as a split
   // sweep's are (its x starts at zero and nothing else writes the resting populations').
   FusedPlan
-  fused_plan(const lbfem_gpu_ctx *ctx, const CgCall &c)
+  fused_plan(lbfem_gpu_ctx *ctx, const CgCall &c)
   {
     FusedPlan f;
     if (ctx->strip || ctx->distorted || c.opk == OPK_LAPLACE)
@@ -854,33 +903,12 @@ namespace
       f.threads = int(std::min<long long>(S::THREADS, (tasks + 31) / 32 * 32));
       return S::GROUP <= g.ncy && f.smem <= FUSED_SMEM && tasks <= (long long)S::MAXT * S::THREADS;
     });
-    for (int s = 0; s < c.nsys && fits; ++s)
+    if (!fits || !fused_resident(ctx, f))
+      return f;
+    for (int s = 0; s < c.nsys; ++s)
       if (!((c.skip >> s) & 1))
         f.sys[f.n++] = s;
     return f;
-  }
-
-  template <int P, bool SEP>
-  cudaError_t
-  fused_launch(const FusedPlan &f, const Geo &geo, const FusedArgs &a, cudaStream_t stream)
-  {
-    // set here and not when a context is made: only the solves of small meshes load the kernel
-    auto kernel = k_cg_fused<P, SEP>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FUSED_SMEM));
-    if (e != cudaSuccess)
-      return e;
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(FusedShape<P>::GROUP * f.n);
-    lc.blockDim = dim3(f.threads);
-    lc.dynamicSmemBytes = f.smem;
-    lc.stream = stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = FusedShape<P>::GROUP;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    lc.attrs = &at;
-    lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, kernel, geo, a);
   }
 
   // The solve c in one launch (plan f): x <- A^{-1} b. ds: the counters of a graph-launched step.
@@ -904,7 +932,10 @@ namespace
     CK(cudaMemsetAsync(state, 0, sizeof(CgState), ctx->stream));
     return with_degree(ctx->P, [&](auto PP) -> int {
       constexpr int P = decltype(PP)::value;
-      CK((f.sep ? fused_launch<P, true>(f, geo, a, ctx->stream) : fused_launch<P, false>(f, geo, a, ctx->stream)));
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t lc = fused_config(f, f.n, FusedShape<P>::GROUP, &at, ctx->stream);
+      CK((f.sep ? cudaLaunchKernelEx(&lc, k_cg_fused<P, true>, geo, a) :
+                  cudaLaunchKernelEx(&lc, k_cg_fused<P, false>, geo, a)));
       ++ctx->launches;
       return LBFEM_OK;
     });
