@@ -276,22 +276,32 @@ namespace
     return LBFEM_OK;
   }
 
+  template <int P, bool TAIL>
+  int
+  set_cg_smem(lbfem_gpu_ctx *ctx)
+  {
+    int st;
+    if ((st = set_smem(ctx, k_cg_start<P, double, double, double, OPK_MASS, TAIL>, cg_smem<P, double>(1))) ||
+        (st = set_smem(ctx, k_cg_p<P, double, OPK_MASS, TAIL>, cg_smem<P, double>(0))) ||
+        (st = set_smem(ctx, k_cg_update<P, double, OPK_MASS, TAIL>, cg_smem<P, double>(0))) ||
+        (st = set_smem(ctx, k_cg_start<P, double, double, double, OPK_TG3, TAIL>, cg_smem<P, double, OPK_TG3>(1))) ||
+        (st = set_smem(ctx, k_cg_p<P, double, OPK_TG3, TAIL>, cg_smem<P, double, OPK_TG3>(0))) ||
+        (st = set_smem(ctx, k_cg_update<P, double, OPK_TG3, TAIL>, cg_smem<P, double, OPK_TG3>(2))) ||
+        (st = set_smem(ctx, k_cg_start<P, double, double, double, OPK_LAPLACE, TAIL>,
+                       cg_smem<P, double, OPK_LAPLACE>(1))) ||
+        (st = set_smem(ctx, k_cg_p<P, double, OPK_LAPLACE, TAIL>, cg_smem<P, double, OPK_LAPLACE>(0))) ||
+        (st = set_smem(ctx, k_cg_update<P, double, OPK_LAPLACE, TAIL>, cg_smem<P, double, OPK_LAPLACE>(2))))
+      return st;
+    return LBFEM_OK;
+  }
+
   template <int P>
   int
   set_smem_attributes(lbfem_gpu_ctx *ctx)
   {
     int st;
     if ((st = set_smem(ctx, k_mass_vmult<P>, cg_smem<P, double>(0))) ||
-        (st = set_smem(ctx, k_cg_start<P, double, double, double>, cg_smem<P, double>(1))) ||
-        (st = set_smem(ctx, k_cg_p<P, double>, cg_smem<P, double>(0))) ||
-        (st = set_smem(ctx, k_cg_update<P, double>, cg_smem<P, double>(0))) ||
-        (st = set_smem(ctx, k_cg_start<P, double, double, double, OPK_TG3>, cg_smem<P, double, OPK_TG3>(1))) ||
-        (st = set_smem(ctx, k_cg_p<P, double, OPK_TG3>, cg_smem<P, double, OPK_TG3>(0))) ||
-        (st = set_smem(ctx, k_cg_update<P, double, OPK_TG3>, cg_smem<P, double, OPK_TG3>(2))) ||
-        (st = set_smem(ctx, k_cg_start<P, double, double, double, OPK_LAPLACE>,
-                       cg_smem<P, double, OPK_LAPLACE>(1))) ||
-        (st = set_smem(ctx, k_cg_p<P, double, OPK_LAPLACE>, cg_smem<P, double, OPK_LAPLACE>(0))) ||
-        (st = set_smem(ctx, k_cg_update<P, double, OPK_LAPLACE>, cg_smem<P, double, OPK_LAPLACE>(2))) ||
+        (st = set_cg_smem<P, false>(ctx)) || (st = set_cg_smem<P, true>(ctx)) ||
         (st = set_smem(ctx, k_cg_start<P, float, float, double>, cg_smem<P, float>(1, true))) ||
         (st = set_smem(ctx, k_window_correct<P>, window_smem<P>())) ||
         (st = set_smem(ctx, kg_stream_pair<P, PAIR_LEELIN>, pair_smem<P, PAIR_LEELIN>())) ||
@@ -742,62 +752,67 @@ namespace
     });
   }
 
-  // r = b - A x_start and the start sums; *n_tiles: the tiles of one system.
-  int
-  cg_launch_start(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int *n_tiles, const CgFinish &fin)
+  // Do the element kernels of a solve end with its sums and scalar work (cg_finish), or do
+  // launches of their own follow them? On a strip always the latter: the sums are added
+  // over the ranks. Else while a launch has few CTAs: the fence at the end of each delays
+  // the next one on its SM, which costs more than two launches from about a wave of
+  // CTAs on (the stack frame of the call takes registers besides). Per step of eight systems,
+  // separate launches and in the kernel: mass Q3 768 CTAs 468 and 453 us, 1216 618 and 628,
+  // 2464 1025 and 1080; mass Q4 952 541 and 514, 1512 724 and 704, 2288 938 and 957; general
+  // TG3 Q1 520 CTAs 134 and 129 us, 952 189 and 193, Q2 672 196 and 201, 1344 299 and 313, 2080
+  // 370 and 389. A single system is solved from the host, where launches cost more: general
+  // TG3 Q2 969 CTAs 1919 and 1858 us, Q1 1298 1902 and 1864, 2688 3604 and 3641.
+  bool
+  tail_solve(const lbfem_gpu_ctx *ctx, const CgCall &c)
   {
-    const Geo geo = geo_of(ctx);
-    return with_degree(ctx->P, [&](auto PP) -> int {
-      constexpr int P = decltype(PP)::value;
-      dim3 grid = tile_grid<P>(ctx->grid);
-      *n_tiles = int(grid.x * grid.y);
-      grid.z = c.nsys;
-      return with_op(c.opk, [&](auto OO) -> int {
-        constexpr int OPK = decltype(OO)::value;
-        k_cg_start<P, double, double, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(OPK == OPK_MASS ? 0 : 1, true), ctx->stream>>>(
-          geo, c.b, c.x_cur, c.x_prev, c.x_new, w.r, c.extrapolate, w.partials, c.sc, c.skip, w.state, fin);
-        LAUNCHED();
-        return LBFEM_OK;
-      });
+    const long long ctas = c.nsys * with_degree(ctx->P, [&](auto PP) -> int {
+      const dim3 t = tile_grid<decltype(PP)::value>(ctx->grid);
+      return int(t.x * t.y);
     });
+    const int most = c.nsys == 1 ? 2400 : ctx->P == 4 && c.opk == OPK_MASS ? 1800 : 1200;
+    return !ctx->strip && ctas <= most;
   }
 
-  // p[1-pi] <- D^{-1} r + beta p[pi] and the sums p.Ap.
+  // One phase of a solve on the element kernels: 0 the start, r = b - A x_start; 1 the
+  // direction, p[1 - pi] <- D^{-1} r + beta p[pi]; 2 the update with p[pi], x += alpha p,
+  // r -= alpha A p. Each with its sums and scalar work (fin), in the kernel or after it.
   int
-  cg_launch_p(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi, const CgFinish &fin)
+  cg_launch(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int phase, int pi, const CgFinish &fin)
   {
     const Geo geo = geo_of(ctx);
-    return with_degree(ctx->P, [&](auto PP) -> int {
+    const bool tail = tail_solve(ctx, c);
+    int n_tiles = 0;
+    int st = with_degree(ctx->P, [&](auto PP) -> int {
       constexpr int P = decltype(PP)::value;
       dim3 grid = tile_grid<P>(ctx->grid);
+      n_tiles = int(grid.x * grid.y);
       grid.z = c.nsys;
-      return with_op(c.opk, [&](auto OO) -> int {
+      auto run = [&](auto OO, auto TT) -> int {
         constexpr int OPK = decltype(OO)::value;
-        k_cg_p<P, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(0), ctx->stream>>>(
-          geo, w.r, w.p[pi], w.p[1 - pi], w.state, w.partials, c.sc, fin);
+        constexpr bool T = decltype(TT)::value;
+        constexpr int own = OPK == OPK_MASS ? 0 : 1;
+        if (phase == 0)
+          k_cg_start<P, double, double, double, OPK, T><<<grid, THREADS, cg_smem<P, double, OPK>(own, true), ctx->stream>>>(
+            geo, c.b, c.x_cur, c.x_prev, c.x_new, w.r, c.extrapolate, w.partials, c.sc, c.skip, w.state, fin);
+        else if (phase == 1)
+          k_cg_p<P, double, OPK, T><<<grid, THREADS, cg_smem<P, double, OPK>(0), ctx->stream>>>(
+            geo, w.r, w.p[pi], w.p[1 - pi], w.state, w.partials, c.sc, fin);
+        else
+          k_cg_update<P, double, OPK, T><<<grid, THREADS, cg_smem<P, double, OPK>(2 * own), ctx->stream>>>(
+            geo, c.x_new, w.r, w.p[pi], w.state, w.partials, c.sc, fin);
         LAUNCHED();
         return LBFEM_OK;
-      });
+      };
+      return with_op(c.opk, [&](auto OO) -> int { return tail ? run(OO, std::true_type()) : run(OO, std::false_type()); });
     });
-  }
-
-  // x += alpha p, r -= alpha A p with p = p[pi], and the sums r.r, r.D^{-1}r.
-  int
-  cg_launch_update(lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c, int pi, const CgFinish &fin)
-  {
-    const Geo geo = geo_of(ctx);
-    return with_degree(ctx->P, [&](auto PP) -> int {
-      constexpr int P = decltype(PP)::value;
-      dim3 grid = tile_grid<P>(ctx->grid);
-      grid.z = c.nsys;
-      return with_op(c.opk, [&](auto OO) -> int {
-        constexpr int OPK = decltype(OO)::value;
-        k_cg_update<P, double, OPK><<<grid, THREADS, cg_smem<P, double, OPK>(OPK == OPK_MASS ? 0 : 2), ctx->stream>>>(
-          geo, c.x_new, w.r, w.p[pi], w.state, w.partials, c.sc, fin);
-        LAUNCHED();
-        return LBFEM_OK;
-      });
-    });
+    if (st || tail)
+      return st;
+    const int nq = (phase == 0 ? 3 : phase) * NM;
+    if ((st = reduce_into(ctx, w.partials, w.sums, n_tiles, nq)) || (st = strip_allreduce(ctx, nq)))
+      return st;
+    k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, phase, fin);
+    LAUNCHED();
+    return LBFEM_OK;
   }
 
   // x <- 0 for the systems flagged by the solver's start (right-hand side exactly zero).
@@ -969,7 +984,7 @@ namespace
     const double tol = c.tol >= 0 ? c.tol : ctx->prm.cg_tolerance;
     const int max_its = c.max_its > 0 ? c.max_its : ctx->prm.cg_max_iterations;
     const int nsys = c.nsys;
-    int n_tiles = 0, st;
+    int st;
     const FusedPlan f = w.state == ctx->d_cg ? fused_plan(ctx, c) : FusedPlan{};
     if (f.n)
       {
@@ -992,30 +1007,16 @@ namespace
     CK(cudaMemsetAsync(w.state, 0, sizeof(CgState), ctx->stream));
     const bool col = column_solve(ctx, w, c);
     CgFinish fin;
-    if (!ctx->strip)
-      {
-        fin.nsys = nsys;
-        fin.cg_tol = tol;
-        fin.max_its = max_its;
-      }
+    fin.nsys = nsys;
+    fin.cg_tol = tol;
+    fin.max_its = max_its;
     CgFinish cnt = fin; // the phases after which the host may read the count of active systems
     cnt.count = 1;
-    // strip mode, the end of a phase: its nq sums, over the ranks, and the scalar work
-    auto phase_end = [&](int phase, int nq) -> int {
-      int s2;
-      if (!ctx->strip)
-        return LBFEM_OK;
-      if ((s2 = reduce_into(ctx, w.partials, w.sums, n_tiles, nq * NM)) || (s2 = strip_allreduce(ctx, nq * NM)))
-        return s2;
-      k_cg_scalars<<<1, 32, 0, ctx->stream>>>(w.state, w.sums, nsys, phase, tol, max_its);
-      LAUNCHED();
-      return LBFEM_OK;
+    auto phase = [&](int ph, int pi, const CgFinish &end) -> int {
+      return col ? col_launch(ctx, w, c, ph, pi, end) : cg_launch(ctx, w, c, ph, pi, end);
     };
-    if (col)
-      st = col_launch(ctx, w, c, 0, 0, cnt);
-    else if (!(st = cg_launch_start(ctx, w, c, &n_tiles, cnt)))
-      st = phase_end(0, 3);
-    if (st || (st = zero_flagged(ctx, c.x_new, w.state, nsys)) || (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
+    if ((st = phase(0, 0, cnt)) || (st = zero_flagged(ctx, c.x_new, w.state, nsys)) ||
+        (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
       return st;
     // the state is read back every few iterations (an iteration of converged systems does nothing)
     const int ahead = ctx->strip || ctx->trace ? 1 : CG_AHEAD;
@@ -1036,19 +1037,10 @@ namespace
             if (ctx->h_cg->n_active == 0)
               break;
           }
-        if (col)
-          {
-            if ((st = col_launch(ctx, w, c, 1, pi, fin)) || (st = col_launch(ctx, w, c, 2, 1 - pi, cnt)))
-              return st;
-            pi = 1 - pi;
-            continue;
-          }
-        if ((st = cg_launch_p(ctx, w, c, pi, fin)) || (st = phase_end(1, 1)))
-          return st;
-        pi = 1 - pi;
-        if ((st = cg_launch_update(ctx, w, c, pi, cnt)) || (st = phase_end(2, 2)) ||
+        if ((st = phase(1, pi, fin)) || (st = phase(2, 1 - pi, cnt)) ||
             (st = strip_exchange(ctx, w.r, nsys, sizeof(double))))
           return st;
+        pi = 1 - pi;
       }
     if (its_out)
       *its_out = ctx->h_cg->total_its;
@@ -1937,17 +1929,15 @@ namespace
     set.ds = ctx->d_stats;
     set.h = h;
     const bool col = column_solve(ctx, w, c);
-    int n_tiles = 0, st;
-    if ((st = col ? col_launch(ctx, w, c, 0, 0, set) : cg_launch_start(ctx, w, c, &n_tiles, set)) ||
-        (st = zero_flagged(ctx, c.x_new, w.state, c.nsys)))
+    auto phase = [&](int ph, int pi, const CgFinish &end) -> int {
+      return col ? col_launch(ctx, w, c, ph, pi, end) : cg_launch(ctx, w, c, ph, pi, end);
+    };
+    int st;
+    if ((st = phase(0, 0, set)) || (st = zero_flagged(ctx, c.x_new, w.state, c.nsys)))
       return st;
     auto iteration = [&](int pi, const CgFinish &end) -> int {
-      int s2;
-      if (col)
-        (s2 = col_launch(ctx, w, c, 1, pi, fin)) || (s2 = col_launch(ctx, w, c, 2, 1 - pi, end));
-      else
-        (s2 = cg_launch_p(ctx, w, c, pi, fin)) || (s2 = cg_launch_update(ctx, w, c, 1 - pi, end));
-      return s2;
+      const int s2 = phase(1, pi, fin);
+      return s2 ? s2 : phase(2, 1 - pi, end);
     };
     return capture_while(
       ctx, h,

@@ -1682,8 +1682,8 @@ namespace lbfem_gpu
     cudaGraphSetConditional(h, go ? 1u : 0u);
   }
 
-  // The rest of a CG phase that its kernel does in its last CTAs (cg_finish); nsys 0: nothing,
-  // the sums are reduced, and added over the ranks of a decomposed mesh, by other launches.
+  // The rest of a CG phase after its kernel's tiles: done by the kernel's last CTAs (cg_finish),
+  // or by launches of their own (k_reduce_partials and k_cg_scalars).
   struct CgFinish
   {
     int nsys = 0;
@@ -1757,18 +1757,18 @@ namespace lbfem_gpu
     cg_system_done(st, *fin, phase);
   }
 
-  // The end of a CG kernel's tile `tile` of nt for system s: its partial sums stored; the
-  // system's last CTA to arrive adds them and does the phase's scalar work. A sums kernel
-  // and a scalar kernel instead cost about 5 us a phase; this costs 2 to 3, the chain of
-  // fences and L2 round trips from the last store to the new scalars (101 x 77 Q4: 431 to
-  // 390 us per step at 8 iterations).
-  template <int NQ, int NT>
+  // The end of a CG kernel's tile `tile` of nt for system s: its partial sums stored; with TAIL
+  // the system's last CTA to arrive adds them and does the phase's scalar work. A sums
+  // kernel and a scalar kernel instead cost about 5 us a phase; this costs 2 to 3, the
+  // chain of fences and L2 round trips from the last store to the new scalars (101 x 77 Q4:
+  // 431 to 390 us per step at 8 iterations), but also a fence at the end of every CTA (tail_solve).
+  template <int NQ, int NT, bool TAIL = true>
   __device__ __forceinline__ void
   cg_finish(double (&part)[NQ], double *__restrict__ partials, CgState *st, int s, int tile, int nt, int phase,
             const CgFinish &fin)
   {
     block_reduce_store_n<NQ, NT>(part, partials + (long long)s * nt, tile, NM * nt);
-    if (!fin.nsys)
+    if constexpr (!TAIL)
       return;
     __shared__ int last;
     if (threadIdx.x == 0)
@@ -1835,7 +1835,7 @@ namespace lbfem_gpu
   // reads it in place, which leaves room for 6 CTAs per SM.
   // Tile (bx, by) of system bz, of an nbx x nby tile grid (the kernel below, and
   // the body of its batched form).
-  template <int P, typename R, typename X, typename A, int OPK>
+  template <int P, typename R, typename X, typename A, int OPK, bool TAIL>
   __device__ __forceinline__ void
   cg_start_tile(const Geo &geo, const R *__restrict__ b, const X *__restrict__ x_cur, const X *__restrict__ x_prev,
                 X *__restrict__ x_new, R *__restrict__ r, int extrapolate, double *__restrict__ partials,
@@ -1857,7 +1857,7 @@ namespace lbfem_gpu
             const int nt = nbx * nby, tile = by * nbx + bx;
             for (int q = 0; q < 3; ++q)
               partials[(long long)(q * NM + s) * nt + tile] = 0.0;
-            if (fin.nsys && tile == 0)
+            if (TAIL && tile == 0)
               {
                 const double v[3] = {0., 0., 0.};
                 cg_scalars(st, s, cg_system(st, s), v, 0, fin.cg_tol, fin.max_its);
@@ -1911,22 +1911,22 @@ namespace lbfem_gpu
     if constexpr (SUMS)
       {
         // partial (quantity k of system s) at [(k*NM + s) * n_tiles + tile]
-        cg_finish<3, THREADS>(part, partials, st, s, by * nbx + bx, nbx * nby, 0, fin);
+        cg_finish<3, THREADS, TAIL>(part, partials, st, s, by * nbx + bx, nbx * nby, 0, fin);
       }
   }
 
-  template <int P, typename R, typename X = R, typename A = R, int OPK = OPK_MASS>
+  template <int P, typename R, typename X = R, typename A = R, int OPK = OPK_MASS, bool TAIL = false>
   __global__ void __launch_bounds__(THREADS, OPK != OPK_MASS ? 2 : sizeof(R) == sizeof(float) ? 8 : 6)
     k_cg_start(const Geo geo, const R *__restrict__ b, const X *__restrict__ x_cur, const X *__restrict__ x_prev,
                X *__restrict__ x_new, R *__restrict__ r, int extrapolate, double *__restrict__ partials,
                const StreamCoef sc, int skip, CgState *st, const CgFinish fin)
   {
-    cg_start_tile<P, R, X, A, OPK>(geo, b, x_cur, x_prev, x_new, r, extrapolate, partials, sc, skip, blockIdx.x,
+    cg_start_tile<P, R, X, A, OPK, TAIL>(geo, b, x_cur, x_prev, x_new, r, extrapolate, partials, sc, skip, blockIdx.x,
                                    blockIdx.y, blockIdx.z, gridDim.x, gridDim.y, st, fin);
   }
 
   // p <- D^{-1} r + beta p (p <- D^{-1} r on the first iteration); partial p.Ap. One system per CTA.
-  template <int P, typename R, int OPK = OPK_MASS>
+  template <int P, typename R, int OPK = OPK_MASS, bool TAIL = false>
   __global__ void __launch_bounds__(THREADS, OPK == OPK_MASS ? 8 : 2)
     k_cg_p(const Geo geo, const R *__restrict__ r, const R *__restrict__ p_in, R *__restrict__ p_out,
            CgState *st, double *__restrict__ partials, const StreamCoef sc, const CgFinish fin)
@@ -1941,7 +1941,7 @@ namespace lbfem_gpu
     const int nt = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
     if (!st->active[s])
       {
-        if (fin.nsys && tile == 0 && threadIdx.x == 0)
+        if (TAIL && tile == 0 && threadIdx.x == 0)
           cg_system_done(st, fin, 1);
         return;
       }
@@ -1973,11 +1973,11 @@ namespace lbfem_gpu
       if (owned_row(gy0 + i, g))
         part[0] += double(pn) * double(Ap);
     });
-    cg_finish<1, THREADS>(part, partials, st, s, tile, nt, 1, fin);
+    cg_finish<1, THREADS, TAIL>(part, partials, st, s, tile, nt, 1, fin);
   }
 
   // v = A p recomputed; x += alpha p, r -= alpha v; partials r.r, r.D^{-1}r. One system per CTA.
-  template <int P, typename R, int OPK = OPK_MASS>
+  template <int P, typename R, int OPK = OPK_MASS, bool TAIL = false>
   __global__ void __launch_bounds__(THREADS, OPK == OPK_MASS ? 8 : 2)
     k_cg_update(const Geo geo, R *__restrict__ x, R *__restrict__ r, const R *__restrict__ p,
                 CgState *st, double *__restrict__ partials, const StreamCoef sc, const CgFinish fin)
@@ -1992,7 +1992,7 @@ namespace lbfem_gpu
     const int nt = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
     if (!st->active[s])
       {
-        if (fin.nsys && tile == 0 && threadIdx.x == 0)
+        if (TAIL && tile == 0 && threadIdx.x == 0)
           cg_system_done(st, fin, 2);
         return;
       }
@@ -2030,7 +2030,7 @@ namespace lbfem_gpu
           part[1] += double(rr) * (cg_inv_jacobi<P, OPK>(geo, maps, gx0, gy0, i, j, image) * double(rr));
         }
     });
-    cg_finish<2, THREADS>(part, partials, st, s, tile, nt, 2, fin);
+    cg_finish<2, THREADS, TAIL>(part, partials, st, s, tile, nt, 2, fin);
   }
 
   // --------------------------- tensor-product window solve (mixed precision)
@@ -2663,19 +2663,23 @@ namespace lbfem_gpu
   }
 
   // The scalar work of one CG phase, one thread per system, from the reduced sums
-  // (sums[q * NM + s]), for a decomposed mesh.
+  // (sums[q * NM + s]), and the loop's condition, where the CG kernels do not end with it.
   __global__ void
-  k_cg_scalars(CgState *st, const double *__restrict__ sums, int nsys, int phase, double cg_tol, int max_its)
+  k_cg_scalars(CgState *st, const double *__restrict__ sums, int phase, const CgFinish fin)
   {
     const int s = threadIdx.x;
-    if (s < nsys)
+    if (s < fin.nsys)
       {
         const double v[3] = {sums[s], phase == 1 ? 0. : sums[NM + s], phase == 0 ? sums[2 * NM + s] : 0.};
-        cg_scalars(st, s, cg_system(st, s), v, phase, cg_tol, max_its);
+        cg_scalars(st, s, cg_system(st, s), v, phase, fin.cg_tol, fin.max_its);
       }
     __syncthreads();
     if (threadIdx.x == 0)
-      cg_count(st, phase);
+      {
+        cg_count(st, phase);
+        if (fin.ds)
+          cg_control(st, fin.ds, fin.h, phase != 0);
+      }
   }
 
   // ------------------------------------------------- device-side step control
