@@ -697,15 +697,22 @@ namespace
 
   // Does the solve run on the column kernels (cg_column.cuh)? A product operator of a whole
   // Cartesian mesh, with the context's own work buffers. From degree 3 on they gain
-  // only on meshes beyond L2: half of a column's x-pass entries are zero there, and
-  // the registers admit fewer threads. FP64 Lee-Lin step, column kernels and element
-  // tiles: 120^2 Q3 409 and 394 us, 60 x 300 Q3 186 and 161, 101 x 77 Q4 461 and 390,
-  // 400^2 Q4 1191 and 1243; against the element tiles with their sums in launches of
-  // their own: 300^2 Q1 113 and 141, 200^2 Q2 380 and 448, 500^2 Q2 1622 and 2106.
+  // only on meshes beyond L2 whose rows fill the column tiles: half of a column's x-pass
+  // entries are zero there, the registers admit fewer threads, and a row of 129 nodes is two
+  // tiles of 65 columns. FP64 Lee-Lin step, column kernels and element tiles: 101 x 77 Q4 461
+  // and 390 us, 220^2 Q3 (440,000 nodes) 1034 and 988, 260^2 Q3 (610,000) 1359 and 1389, 340^2 Q3
+  // 1894 and 2137; 1.5 million nodes, 145 columns Q3 (57% of the tiles) 3612 and 3167, 193 Q3
+  // (75%) 2811 and 2897, 319 Q3 (83%) 2879 and 2998, 129 Q4 (50%) 4296 and 3592, 193 Q4 (75%)
+  // 3391 and 3373, 321 Q4 (84%) 3133 and 3157. At degrees 1 and 2 they win at every size and
+  // width measured: 128 x 2325 Q1 (129 columns) 633 and 705, 300^2 Q1 442 and 530, 64 x 1162 Q2
+  // 1020 and 1058, 500^2 Q2 1622 and 2106.
   bool
   column_solve(const lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c)
   {
-    if (ctx->strip || c.opk == OPK_LAPLACE || w.state != ctx->d_cg || (ctx->P > 2 && ctx->grid.N < 1000000))
+    if (ctx->strip || c.opk == OPK_LAPLACE || w.state != ctx->d_cg)
+      return false;
+    const int tiles = (ctx->grid.nfx + 127) / 128; // of a row (col_width)
+    if (ctx->P > 2 && (ctx->grid.N < 1000000 || 4 * ctx->grid.nfx < 3 * 128 * tiles))
       return false;
     for (int s = 0; s < c.nsys; ++s)
       if (c.opk == OPK_TG3 && !((c.skip >> s) & 1) && c.sc.kxy[s] != 0.)
