@@ -765,7 +765,8 @@ namespace
   // the next one on its SM, which costs more than two launches from about a wave of
   // CTAs on (the stack frame of the call takes registers besides). Per step of eight systems,
   // separate launches and in the kernel: mass Q3 768 CTAs 468 and 453 us, 1216 618 and 628,
-  // 2464 1025 and 1080; mass Q4 952 541 and 514, 1512 724 and 704, 2288 938 and 957; general
+  // 2464 1025 and 1080; mass Q4 952 541 and 514, 1512 724 and 704, 64 x 291 cells 1960 878 and
+  // 847, 2288 938 and 957; general
   // TG3 Q1 520 CTAs 134 and 129 us, 952 189 and 193, Q2 672 196 and 201, 1344 299 and 313, 2080
   // 370 and 389. A single system is solved from the host, where launches cost more: general
   // TG3 Q2 969 CTAs 1919 and 1858 us, Q1 1298 1902 and 1864, 2688 3604 and 3641.
@@ -776,7 +777,7 @@ namespace
       const dim3 t = tile_grid<decltype(PP)::value>(ctx->grid);
       return int(t.x * t.y);
     });
-    const int most = c.nsys == 1 ? 2400 : ctx->P == 4 && c.opk == OPK_MASS ? 1800 : 1200;
+    const int most = c.nsys == 1 ? 2400 : ctx->P == 4 && c.opk == OPK_MASS ? 2200 : 1200;
     return !ctx->strip && ctas <= most;
   }
 

@@ -24,9 +24,9 @@ def _tiles(nx, ny, p):
     return -(-(p * nx + 1) // w) * -(-(p * ny + 1) // 24)
 
 
-# 8 x 150 and 8 x 152 CTAs at p = 1 .. 3; at p = 4 the mass changes at 1800 (225 and 228 tiles)
-STEPS = [("tg2", 3, 199, 119, 150, True), ("tg2", 3, 160, 150, 152, False), ("tg2", 4, 149, 131, 220, True),
-         ("tg2", 4, 149, 137, 230, False), ("tg3", 1, 639, 359, 150, True), ("tg3", 1, 511, 455, 152, False),
+# 8 x 150 and 8 x 152 CTAs at p = 1 .. 3; at p = 4 the mass changes at 2200 (275 and 280 tiles)
+STEPS = [("tg2", 3, 199, 119, 150, True), ("tg2", 3, 160, 150, 152, False), ("tg2", 4, 164, 149, 275, True),
+         ("tg2", 4, 149, 167, 280, False), ("tg3", 1, 639, 359, 150, True), ("tg3", 1, 511, 455, 152, False),
          ("tg3", 2, 159, 359, 150, True), ("tg3", 2, 255, 227, 152, False), ("tg3", 3, 199, 119, 150, True),
          ("tg3", 4, 119, 110, 152, False)]
 
