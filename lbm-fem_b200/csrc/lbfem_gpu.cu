@@ -87,6 +87,7 @@ struct lbfem_gpu_ctx
   int64_t graph_epoch = 0; // counts the invalidations of the step graphs (batch graphs embed them)
   cudaStream_t cap = nullptr;     // captures the loop bodies
   DevStats *d_stats = nullptr, *h_stats = nullptr;
+  int beside = 1; // instances whose steps are recorded into one batch graph with this one's, itself included
   // the tuned tile shape of the FP32 streaming kernel (tune_pair) and the times it was chosen by
   int pair_shape = 0;
   bool pair_tuned = false;
@@ -366,12 +367,19 @@ namespace
   // Measured, FP64 lumped step with 1 / 2 / 4 / 8 CTAs per tile: 18 tiles 63 / 47 /
   // 39 / 34 us, 55 tiles 63 / 47 / 41 / 46, 96 tiles 65 / 54 / 59 / 61, 260 tiles 73 /
   // 80 / 92 / 113; FP32 pairs with 1 / 2 / 4: 17 tiles 30 / 26 / 24 us, 152 tiles 43 /
-  // 47 / 52.
+  // 47 / 52. In a batch graph the instances' branches start one after the other and about 8 of
+  // them stream at once, so a tile counts that often there. Batches, lumped Lee-Lin FP64,
+  // unsplit / as if alone / counted 4 / 8 / 16 times: 64 of 64^2 Q1 360 / 401 / 405 / 344 / 328
+  // us per step, 8 of 128^2 Q1 81 / 92 / 78 / 71 / 72, 16 of 128^2 Q2 269 / 312 / 254 / 255 / 254,
+  // 32 of 200^2 Q1 383 / 543 / 388 / 356 / 357; iterated lumping, 32 of 200^2 Q1 588 / 775 / 621 /
+  // 588 / 589; mixed Bardow, 8 of 128^2 Q1 80 / 70 / 69 / 74 / 73, 64 of 64^2 Q1 391 / 364 /
+  // 363 / 327 / 324.
   int
-  split_of(const dim3 &tiles, int most)
+  split_of(const lbfem_gpu_ctx *ctx, const dim3 &tiles, int most)
   {
+    const long long n = (long long)tiles.x * tiles.y * std::min(ctx->beside, 8);
     int z = 1;
-    while (z < most && int(tiles.x * tiles.y) * 2 * z <= 2 * 148)
+    while (z < most && n * 2 * z <= 2 * 148)
       z *= 2;
     return z;
   }
@@ -393,7 +401,7 @@ namespace
     return with_degree(ctx->P, [&](auto PP) -> int {
       constexpr int P = decltype(PP)::value;
       dim3 grid = tile_grid<P>(ctx->grid);
-      grid.z = split_of(grid, NM);
+      grid.z = split_of(ctx, grid, NM);
       auto run = [&](auto MODE, auto SPLIT) -> cudaError_t {
         constexpr int M = decltype(MODE)::value;
         auto kernel = k_advection<P, M, R, decltype(SPLIT)::value>;
@@ -439,7 +447,7 @@ namespace
         using S = decltype(SS);
         using T = Tile<P, S>;
         dim3 grid((ctx->grid.nfx + T::TX - 1) / T::TX, (ctx->grid.nfy + T::TY - 1) / T::TY);
-        grid.z = split_of(grid, 4);
+        grid.z = split_of(ctx, grid, 4);
         auto run = [&](auto MODE, auto SPLIT) -> cudaError_t {
           constexpr int M = decltype(MODE)::value;
           auto kernel = k_stream_pair<P, M, S, decltype(SPLIT)::value>;
@@ -3977,7 +3985,10 @@ namespace
         ce = cudaStreamWaitEvent(c->stream, b->fork, 0);
         if (ce != cudaSuccess)
           break;
-        if ((st = record_step(c, &e.fixed[k], &e.body[k])))
+        c->beside = int(b->ctxs.size());
+        st = record_step(c, &e.fixed[k], &e.body[k]);
+        c->beside = 1;
+        if (st)
           {
             batch_fail(b, st, "instance %zu: %s", k, c->err.c_str());
             break;
