@@ -18,10 +18,10 @@
 // direction. Sums are fixed-order: a warp's tree, then a tree over the warps of
 // all CTAs, the same on every thread.
 //
-// A form with more CTAs than a cluster holds, meeting at counters in global
-// memory, was measured and dropped: there a sum took 6 to 10 us (the partial
-// sums and halo rows are lines that every SM writes and reads), no less than the
-// launches it replaced.
+// A form with more CTAs than a cluster holds, meeting at counters in global memory,
+// was measured and left out: a sum took 6 to 10 us there (the partial sums and
+// halo rows are lines that every SM writes and reads), and its waits hold only if
+// every CTA of the solve is resident, beside whatever else the GPU runs.
 #pragma once
 
 #include "operators.cuh"
