@@ -9,8 +9,8 @@
 // start at cell boundaries.
 //
 // The element-tile form of these kernels (k_cg_start / _p / _update, kept for the general
-// TG3 and Laplace operators, strips, the solve without allocation, and the meshes of degrees
-// 3 and 4 on which it is the faster one) spends
+// TG3 and Laplace operators, strips, the solve without allocation, and the meshes on which
+// it is the faster one) spends
 // 160 instructions per node, most of them on index maps and staging, and leaves
 // lanes idle in both passes; it was bound by issue and latency on L2-resident
 // meshes (13.5 and 21.7 us per launch on 405 x 309 Q4 nodes, 8 systems, whose data

@@ -703,37 +703,49 @@ namespace
       }
   }
 
-  // Does the solve run on the column kernels (cg_column.cuh)? A product operator of a whole
-  // Cartesian mesh, with the context's own work buffers. From degree 3 on they gain
-  // only on meshes beyond L2 whose rows fill the column tiles: half of a column's x-pass
-  // entries are zero there, the registers admit fewer threads, and a row of 129 nodes is two
-  // tiles of 65 columns. FP64 Lee-Lin step, column kernels and element tiles: 101 x 77 Q4 461
-  // and 390 us, 220^2 Q3 (440,000 nodes) 1034 and 988, 260^2 Q3 (610,000) 1359 and 1389, 340^2 Q3
-  // 1894 and 2137; 1.5 million nodes, 145 columns Q3 (57% of the tiles) 3612 and 3167, 193 Q3
-  // (75%) 2811 and 2897, 319 Q3 (83%) 2879 and 2998, 129 Q4 (50%) 4296 and 3592, 193 Q4 (75%)
-  // 3391 and 3373, 321 Q4 (84%) 3133 and 3157. At degrees 1 and 2 they win at every size and
-  // width measured: 128 x 2325 Q1 (129 columns) 633 and 705, 300^2 Q1 442 and 530, 64 x 1162 Q2
-  // 1020 and 1058, 500^2 Q2 1622 and 2106.
-  bool
-  column_solve(const lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c)
-  {
-    if (ctx->strip || c.opk == OPK_LAPLACE || w.state != ctx->d_cg)
-      return false;
-    const int tiles = (ctx->grid.nfx + 127) / 128; // of a row (col_width)
-    if (ctx->P > 2 && (ctx->grid.N < 1000000 || 4 * ctx->grid.nfx < 3 * 128 * tiles))
-      return false;
-    for (int s = 0; s < c.nsys; ++s)
-      if (c.opk == OPK_TG3 && !((c.skip >> s) & 1) && c.sc.kxy[s] != 0.)
-        return false;
-    return true;
-  }
-
   template <int P>
   dim3
   col_grid(const Grid &g, int nsys)
   {
     const int tw = col_width(g.nfx);
     return dim3((g.nfx + tw - 1) / tw, (g.nfy + ColShape<P>::RT - 1) / ColShape<P>::RT, nsys);
+  }
+
+  // Does the solve run on the column kernels (cg_column.cuh)? A product operator of a whole
+  // Cartesian mesh, with the context's own work buffers. From degree 3 on they gain
+  // only on meshes beyond L2: half of a column's x-pass entries are zero there and the
+  // registers admit fewer threads. FP64 Lee-Lin step, column kernels and element tiles:
+  // 101 x 77 Q4 461 and 390 us, 220^2 Q3 (440,000 nodes) 1034 and 988, 260^2 Q3 (610,000) 1359 and
+  // 1389, 340^2 Q3 1894 and 2137.
+  // The mass matrix's element form is cheap enough to win where the rows leave lanes of the column
+  // tiles idle. From degree 3 on below three quarters full: 1.5 million nodes, 145 columns Q3
+  // (57%: two tiles of 73) 3612 and 3167, 193 Q3 (75%) 2811 and 2897, 319 Q3 (83%) 2879 and 2998,
+  // 129 Q4 (50%) 4296 and 3592, 193 Q4 (75%) 3391 and 3373. At degrees 1 and 2 on meshes no wider
+  // than an element tile, beyond a wave of column CTAs (before, latency decides): 33 columns
+  // Q1, 8 systems, 912 CTAs 319 and 375, 1824 492 and 462, 18184 3683 and 2788; 63 Q2 480 CTAs 551
+  // and 607, 960 697 and 638; one system, 33 Q1 569 CTAs 882 and 1027, 17 Q1 1103 1358 and
+  // 1157. Wider ones gain at every size: 128 x 2325 Q1 633 and 705, 64 x 1162 Q2 1020 and 1058,
+  // 300^2 Q1 442 and 530, 500^2 Q2 1622 and 2106. So does split TG3 at every width: 33 columns Q1
+  // 608 and 796, 4818 and 6130, 145 Q3 6285 and 8868.
+  bool
+  column_solve(const lbfem_gpu_ctx *ctx, const CgScratch<double> &w, const CgCall &c)
+  {
+    const Grid &g = ctx->grid;
+    if (ctx->strip || c.opk == OPK_LAPLACE || w.state != ctx->d_cg || (ctx->P > 2 && g.N < 1000000))
+      return false;
+    dim3 cols;
+    with_degree(ctx->P, [&](auto PP) -> int {
+      cols = col_grid<decltype(PP)::value>(g, 1);
+      return 0;
+    });
+    if (c.opk == OPK_MASS && ctx->P > 2 && 4 * g.nfx < 3 * 128 * int(cols.x))
+      return false;
+    if (c.opk == OPK_MASS && ctx->P <= 2 && g.nfx <= 64 && (long long)c.nsys * cols.y > 950)
+      return false;
+    for (int s = 0; s < c.nsys; ++s)
+      if (c.opk == OPK_TG3 && !((c.skip >> s) & 1) && c.sc.kxy[s] != 0.)
+        return false;
+    return true;
   }
 
   // One phase of a solve on the column kernels: 0 the start, 1 the direction p[1 - pi] from

@@ -1,6 +1,6 @@
-"""The column kernels of the FP64 CG at degrees 3 and 4, which take meshes of 10^6 nodes or more
-whose rows fill the tiles of 128 columns to three quarters (column_solve), against the
-oracle: exactly 10^6 nodes and just below, widths on both sides of the three quarters,
+"""The column kernels of the FP64 CG at degrees 3 and 4, which take meshes of 10^6 nodes or more,
+for the mass matrix those whose rows fill the tiles of 128 columns to three quarters
+(column_solve), against the oracle: exactly 10^6 nodes and just below, widths on both sides of the three quarters,
 last tiles of one row, walls and periodic axes, the mass matrix and both
 axis-parallel TG3 matrices. A step's launches per CG iteration tell which form ran: 2 of the
 column kernels, 6 of the element kernels at these sizes.
@@ -20,7 +20,7 @@ from lbfem_gpu import cases, make_params
 pytestmark = pytest.mark.gpu
 
 TOL = 1e-13
-# (flow, nx, ny, p, column kernels); tiles of 18 rows at p = 3, of 16 at p = 4
+# (flow, nx, ny, p, column kernels for the mass matrix); tiles of 18 rows at p = 3, of 16 at p = 4
 SIZES = [("tgv", 333, 333, 3, True), ("cavity", 333, 332, 3, False), ("cavity", 346, 336, 3, True),
          ("couette", 42, 2700, 3, True), ("couette", 64, 1730, 3, True), ("couette", 63, 1760, 3, False),
          ("tgv", 250, 250, 4, True), ("couette", 48, 1300, 4, True), ("cavity", 47, 1330, 4, False),
